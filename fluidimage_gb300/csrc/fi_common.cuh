@@ -87,6 +87,64 @@ __device__ __forceinline__ int load_px_int(const void* im, int dtype, int64_t id
                           : (int)__ldg(reinterpret_cast<const uint16_t*>(im) + idx);
 }
 
+// Minimum of 16 bytes of pixels (u8: 16, u16: 8, f32: 4 values).
+__device__ __forceinline__ float min16(uint4 v, int dtype) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  if (dtype == FI_F32) {
+    return fminf(fminf(__uint_as_float(w[0]), __uint_as_float(w[1])),
+                 fminf(__uint_as_float(w[2]), __uint_as_float(w[3])));
+  }
+  uint32_t m = 0xffffffffu;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (dtype == FI_U16) {
+      m = min(m, min(w[k] & 0xffffu, w[k] >> 16));
+    } else {
+      m = min(m, min(min(w[k] & 0xffu, (w[k] >> 8) & 0xffu),
+                     min((w[k] >> 16) & 0xffu, w[k] >> 24)));
+    }
+  }
+  return (float)m;  // exact: below 2^16
+}
+
+// The minima (m0, m1) of two images of `count` pixels over thread `tid` of `stride`:
+// 16-byte loads, four of each image in flight, when both images are 16-byte aligned.
+__device__ __forceinline__ void min_of_pair(const void* im0, const void* im1, int dtype,
+                                            int64_t count, int64_t tid, int64_t stride,
+                                            float& m0, float& m1) {
+  const int esize = (dtype == FI_U8) ? 1 : (dtype == FI_U16 ? 2 : 4);
+  int64_t vec = 0;  // pixels read by 16-byte loads
+  if ((((uintptr_t)im0 | (uintptr_t)im1) & 15) == 0) {
+    const int per = 16 / esize;
+    const int64_t nv = count / per;
+    const uint4* a = reinterpret_cast<const uint4*>(im0);
+    const uint4* b = reinterpret_cast<const uint4*>(im1);
+    int64_t i = tid;
+    for (; i + 3 * stride < nv; i += 4 * stride) {
+      uint4 va[4], vb[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        va[k] = __ldg(a + i + k * stride);
+        vb[k] = __ldg(b + i + k * stride);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        m0 = fminf(m0, min16(va[k], dtype));
+        m1 = fminf(m1, min16(vb[k], dtype));
+      }
+    }
+    for (; i < nv; i += stride) {
+      m0 = fminf(m0, min16(__ldg(a + i), dtype));
+      m1 = fminf(m1, min16(__ldg(b + i), dtype));
+    }
+    vec = nv * per;
+  }
+  for (int64_t i = vec + tid; i < count; i += stride) {
+    m0 = fminf(m0, load_px(im0, dtype, i));
+    m1 = fminf(m1, load_px(im1, dtype, i));
+  }
+}
+
 // Order-preserving float <-> uint32 keys (for atomicMin over floats).
 __device__ __forceinline__ uint32_t float_to_key(float f) {
   uint32_t u = __float_as_uint(f);

@@ -112,48 +112,12 @@ __global__ void k_min_init(uint32_t* keys) {
   if (threadIdx.x < 2) keys[threadIdx.x] = 0xFFFFFFFFu;
 }
 
-// Minimum of 16 bytes of pixels (u8: 16, u16: 8, f32: 4 values).
-__device__ __forceinline__ float min16(uint4 v, int dtype) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-  if (dtype == FI_F32) {
-    return fminf(fminf(__uint_as_float(w[0]), __uint_as_float(w[1])),
-                 fminf(__uint_as_float(w[2]), __uint_as_float(w[3])));
-  }
-  uint32_t m = 0xffffffffu;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (dtype == FI_U16) {
-      m = min(m, min(w[k] & 0xffffu, w[k] >> 16));
-    } else {
-      m = min(m, min(min(w[k] & 0xffu, (w[k] >> 8) & 0xffu),
-                     min((w[k] >> 16) & 0xffu, w[k] >> 24)));
-    }
-  }
-  return (float)m;  // exact: below 2^16
-}
-
 __global__ void k_images_min(const void* im0, const void* im1, int dtype, int64_t count,
                              uint32_t* keys) {
   float m0 = INFINITY, m1 = INFINITY;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const int esize = (dtype == FI_U8) ? 1 : (dtype == FI_U16 ? 2 : 4);
-  int64_t vec = 0;  // pixels read by 16-byte loads (both images 16-byte aligned)
-  if ((((uintptr_t)im0 | (uintptr_t)im1) & 15) == 0) {
-    const int per = 16 / esize;
-    const int64_t nv = count / per;
-    const uint4* a = reinterpret_cast<const uint4*>(im0);
-    const uint4* b = reinterpret_cast<const uint4*>(im1);
-    for (int64_t i = tid; i < nv; i += stride) {
-      m0 = fminf(m0, min16(__ldg(a + i), dtype));
-      m1 = fminf(m1, min16(__ldg(b + i), dtype));
-    }
-    vec = nv * per;
-  }
-  for (int64_t i = vec + tid; i < count; i += stride) {
-    m0 = fminf(m0, load_px(im0, dtype, i));
-    m1 = fminf(m1, load_px(im1, dtype, i));
-  }
+  min_of_pair(im0, im1, dtype, count, tid, stride, m0, m1);
   for (int o = 16; o > 0; o >>= 1) {
     m0 = fminf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
     m1 = fminf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
