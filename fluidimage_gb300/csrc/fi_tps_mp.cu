@@ -1539,21 +1539,44 @@ extern "C" int fi_tps_solve_mp(const fi_tps_plan* plan, int nb_subdom, int max_m
              "fi_tps_solve_mp: matrices must be 16-byte aligned");
   FI_REQUIRE(((uintptr_t)phi_table2 & 7) == 0, "fi_tps_solve_mp: phi_table2 must be 8-byte aligned");
   const int N = max_members > 4 ? max_members : 4;
-  // 16 warps per subdomain when the subdomains fit in one wave of blocks (shorter
-  // latency per subdomain), else two blocks of 8 warps per SM
   int dev = 0, nsm = 0;
   FI_CUDA_TRY(cudaGetDevice(&dev));
   FI_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const bool wide = nb_subdom <= nsm;
-  const MpLayout lay(N, wide ? 16 : 8);
-  const size_t smem = lay.bytes;
+  // 16 warps per subdomain when the subdomains fit in one wave of blocks (shorter
+  // latency per subdomain) or when the shared memory of a subdomain leaves room for
+  // only one narrow block per SM (more than ~460 centres: 8 warps per SM would do all
+  // the work; 992 subdomains of ~500 centres: 7.2 ms so, 6.5 ms with 16 warps);
+  // else two blocks of 8 warps per SM
+  static SmemLimit limit_wide, limit_narrow;
+  size_t smem = MpLayout(N, 8).bytes;
+  int per_sm = 0;  // resident narrow blocks per SM
+  bool wide = nb_subdom <= nsm;
+  if (!wide && smem <= 220 * 1024) {
+    FI_CUDA_TRY(raise_smem_limit(k_tps_solve_mp<256>, smem, limit_narrow));
+    // queried once per device and size: the call sits between the host's readback and
+    // the launch
+    static size_t occ_smem[FI_SMEM_DEVICES] = {};
+    static int occ_blocks[FI_SMEM_DEVICES] = {};
+    per_sm = -1;
+    {
+      std::lock_guard<std::mutex> lock(smem_limit_mutex());
+      if (dev < FI_SMEM_DEVICES && occ_smem[dev] == smem) per_sm = occ_blocks[dev];
+    }
+    if (per_sm < 0) {
+      FI_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tps_solve_mp<256>,
+                                                                256, smem));
+      std::lock_guard<std::mutex> lock(smem_limit_mutex());
+      if (dev < FI_SMEM_DEVICES) {
+        occ_smem[dev] = smem;
+        occ_blocks[dev] = per_sm;
+      }
+    }
+    wide = per_sm < 2 && MpLayout(N, 16).bytes <= 220 * 1024;
+  }
+  if (wide) smem = MpLayout(N, 16).bytes;
   FI_REQUIRE(smem <= 220 * 1024, "fi_tps_solve_mp: subdomain of %d vectors too large",
              max_members);
-  static SmemLimit limit_wide, limit_narrow;
-  if (wide)
-    FI_CUDA_TRY(raise_smem_limit(k_tps_solve_mp<512>, smem, limit_wide));
-  else
-    FI_CUDA_TRY(raise_smem_limit(k_tps_solve_mp<256>, smem, limit_narrow));
+  if (wide) FI_CUDA_TRY(raise_smem_limit(k_tps_solve_mp<512>, smem, limit_wide));
   if (wide) {
     // clusters of S CTAs per subdomain while the subdomains leave SMs idle
     const int S = (4 * nb_subdom <= nsm) ? 4 : (2 * nb_subdom <= nsm) ? 2 : 1;
@@ -1576,24 +1599,6 @@ extern "C" int fi_tps_solve_mp(const fi_tps_plan* plan, int nb_subdom, int max_m
                                    use_threshold, w_offsets, weights, smoothed_x, smoothed_y,
                                    iters, nfixed, status, max_udiff, sweeps, order, 60, N));
   } else {
-    // resident narrow blocks per SM for this shared-memory size (queried once per
-    // device and size: the call sits between the host's readback and the launch)
-    static size_t occ_smem[FI_SMEM_DEVICES] = {};
-    static int occ_blocks[FI_SMEM_DEVICES] = {};
-    int per_sm = -1;
-    {
-      std::lock_guard<std::mutex> lock(smem_limit_mutex());
-      if (dev < FI_SMEM_DEVICES && occ_smem[dev] == smem) per_sm = occ_blocks[dev];
-    }
-    if (per_sm < 0) {
-      FI_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tps_solve_mp<256>,
-                                                                256, smem));
-      std::lock_guard<std::mutex> lock(smem_limit_mutex());
-      if (dev < FI_SMEM_DEVICES) {
-        occ_smem[dev] = smem;
-        occ_blocks[dev] = per_sm;
-      }
-    }
     const int slots = per_sm * nsm;
     const int head = (order != nullptr && slots > 0 && nb_subdom > slots &&
                       nb_subdom < 2 * slots) ? slots : nb_subdom;
