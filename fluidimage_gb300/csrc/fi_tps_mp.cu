@@ -12,9 +12,10 @@
 // compact WY form of Q; the projection cancels the large affine part of K, so it
 // needs more than FP32: Y = A V and B are computed in double-float (pairs of floats,
 // error-free products and sums on the FP32 pipe, ~48 bits), the O(n) parts and C in
-// FP64.  B is kept as (hi, lo) pairs and its FP32 rounding is factorised (tiled
-// Cholesky).  z is refined in double-float: rho = g - B z on the FP32 pipe
-// (error-free products and sums), then an FP32 Cholesky solve for the correction.
+// FP64.  B is kept as (hi, lo) pairs and its high terms are factorised (tiled Cholesky
+// on the tensor cores, FP16 pairs with FP32 accumulation).  z is refined in double-float:
+// rho = g - B z on the FP32 pipe (error-free products and sums), then a solve with the
+// factor for the correction.
 // Each sweep contracts the error ~1e3-1e4 times; refinement stops when the
 // predicted remaining error is below 1e-10 of z, or when it stagnates (then it must
 // be below 1e-9).  A subdomain that does not converge (or whose P has rank < 3, or
@@ -27,6 +28,7 @@
 // subdomain's centres lie on a grid of the lattice, the block keeps the (hi, lo)
 // values of every grid offset in shared memory (the same table entries).
 #include <cooperative_groups.h>
+#include <cuda_fp16.h>
 
 #include <climits>
 #include <cmath>
@@ -70,72 +72,94 @@ __global__ void k_phi_table2(float2* table, int64_t count) {
 }
 
 // ------------------------------------------------------------------ block helpers
-template <int NT>
-__device__ __forceinline__ double bsum(double v, double* sh) {
+// FP64 is narrow on this GPU (an instruction holds its scheduler's FP64 unit for ~70
+// cycles), so the block-wide steps below keep FP64 additions, and scalar FP64 work on
+// every thread, to a minimum.
+
+// Sums of K values over the block, returned to every thread in out[K] (shared).  The
+// warps reduce-scatter: with P = K rounded up to a power of two, P - 1 + 5 - log2 P
+// additions instead of 5 K.  sh: BLOCK_SUMS doubles.
+constexpr int BLOCK_SUMS = 16 * 16;
+template <int NT, int K>
+__device__ __forceinline__ void block_sums(const double (&v)[K], double* sh, double* out) {
+  constexpr int NW = NT / 32;
+  constexpr int P = K <= 1 ? 1 : K <= 2 ? 2 : K <= 4 ? 4 : K <= 8 ? 8 : 16;
+  static_assert(K <= 16 && NW <= 16, "block_sums: sh");
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (lane == 0) sh[wid] = v;
+  double w[P];
+#pragma unroll
+  for (int k = 0; k < P; ++k) w[k] = k < K ? v[k < K ? k : 0] : 0.0;
+#pragma unroll
+  for (int st = 0; st < 5; ++st) {
+    const int o = 16 >> st, len = P >> (st + 1);
+    if (len > 0) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int k = 0; k < len; ++k) {
+        const double send = up ? w[k] : w[k + len], keep = up ? w[k + len] : w[k];
+        w[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    } else {
+      w[0] += __shfl_xor_sync(0xffffffffu, w[0], o);
+    }
+  }
+  constexpr int PARTS = 32 / P;  // lanes that end with the same value
+  if (lane % PARTS == 0) sh[wid * P + lane / PARTS] = w[0];
   __syncthreads();
   if (wid == 0) {
-    v = lane < NT / 32 ? sh[lane] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) sh[32] = v;
+    const int idx = lane % P;
+    double t = 0.0;
+    for (int q = lane / P; q < NW; q += PARTS) t += sh[q * P + idx];
+#pragma unroll
+    for (int o = P; o < 32; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane < K) out[lane] = t;
   }
   __syncthreads();
-  v = sh[32];
-  __syncthreads();
-  return v;
 }
 
+// Largest of a and of b (non-negative floats, as their bits: a NaN is the largest) over
+// the block.
 template <int NT>
-__device__ __forceinline__ double2 bsum2(double2 v, double* sh) {
+__device__ __forceinline__ float2 block_max2(float a, float b, double* sh) {
+  constexpr int NW = NT / 32;
+  unsigned* u = reinterpret_cast<unsigned*>(sh);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int o = 16; o > 0; o >>= 1) {
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-  }
+  const unsigned full = 0xffffffffu;
+  const unsigned wa = __reduce_max_sync(full, __float_as_uint(a));
+  const unsigned wb = __reduce_max_sync(full, __float_as_uint(b));
   if (lane == 0) {
-    sh[2 * wid] = v.x;
-    sh[2 * wid + 1] = v.y;
+    u[wid] = wa;
+    u[NW + wid] = wb;
   }
   __syncthreads();
-  if (wid == 0) {
-    v.x = lane < NT / 32 ? sh[2 * lane] : 0.0;
-    v.y = lane < NT / 32 ? sh[2 * lane + 1] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) {
-      v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-      v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-    }
-    if (lane == 0) {
-      sh[64] = v.x;
-      sh[65] = v.y;
-    }
-  }
+  const unsigned ra = __reduce_max_sync(full, lane < NW ? u[lane] : 0u);
+  const unsigned rb = __reduce_max_sync(full, lane < NW ? u[NW + lane] : 0u);
   __syncthreads();
-  v.x = sh[64];
-  v.y = sh[65];
-  __syncthreads();
-  return v;
+  return make_float2(__uint_as_float(ra), __uint_as_float(rb));
 }
 
+// Largest of a non-negative double over the warp, by its bits.
+__device__ __forceinline__ double warp_max_pos(double v) {
+  const unsigned full = 0xffffffffu;
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned mh = __reduce_max_sync(full, hi);
+  const unsigned ml = __reduce_max_sync(full, hi == mh ? lo : 0u);
+  return __hiloint2double((int)mh, (int)ml);
+}
 template <int NT>
-__device__ __forceinline__ double bmax(double v, double* sh) {
+__device__ __forceinline__ double block_max_pos(double v, double* sh) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  v = warp_max_pos(v);
   if (lane == 0) sh[wid] = v;
   __syncthreads();
-  if (wid == 0) {
-    v = lane < NT / 32 ? sh[lane] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (lane == 0) sh[32] = v;
-  }
-  __syncthreads();
-  v = sh[32];
+  v = warp_max_pos(lane < NT / 32 ? sh[lane] : 0.0);
   __syncthreads();
   return v;
 }
 
-constexpr int TS = 36;  // row stride (floats) of the 32 x 32 shared tiles: float4-aligned rows
+// bytes of a block's panel: the chunk sums of Y, the projection's per-warp tiles, then
+// the factorisation's staging and the tiles of small subdomains
+__host__ __device__ constexpr size_t panel_bytes(int warps) { return (size_t)(2 + warps) * 4608; }
 
 // Start moving [p, p + bytes) from memory into L2 without waiting for it (bulk
 // prefetch by the copy engine; p 16-byte aligned, bytes a multiple of 16).
@@ -152,7 +176,7 @@ __device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes) {
 // (contiguous, 32 ld bytes per column) while it works on the current one, so that
 // its loads wait on L2 rather than on memory.  rho is rounded to float.
 template <int NT>
-__device__ void residual_df2(const float2* __restrict__ B, int m, int ld, const float2* zx,
+__device__ __noinline__ void residual_df2(const float2* __restrict__ B, int m, int ld, const float2* zx,
                              const float2* zy, const float2* gx, const float2* gy, float* rx,
                              float* ry) {
   constexpr int NW = NT / 32;
@@ -248,490 +272,482 @@ __device__ void residual_df2(const float2* __restrict__ B, int m, int ld, const 
   __syncthreads();
 }
 
-// Apply H_k = I - tau_k v_k v_k^T (k in order) to the two vectors x, y (length n);
-// v_k is row k of V (row stride vstride).
-template <int NT, bool REVERSE>
-__device__ void apply_reflectors2(const double* V, int vstride, const double* tau, int n,
-                                  double* x, double* y, double* sh) {
-  for (int kk = 0; kk < 3; ++kk) {
-    const int k = REVERSE ? 2 - kk : kk;
-    const double* v = V + (int64_t)k * vstride;
-    double2 d = make_double2(0.0, 0.0);
-    for (int i = threadIdx.x; i < n; i += NT) {
-      d.x += v[i] * x[i];
-      d.y += v[i] * y[i];
-    }
-    d = bsum2<NT>(d, sh);
-    const double cx = tau[k] * d.x, cy = tau[k] * d.y;
-    for (int i = threadIdx.x; i < n; i += NT) {
-      x[i] -= cx * v[i];
-      y[i] -= cy * v[i];
-    }
-    __syncthreads();
-  }
-}
+// ---- Cholesky preconditioner on the tensor cores ------------------------------------
+// The factor of D B D (D: powers of two that bring the diagonal into [1, 4)) by 32 x 32
+// tiles, each kept as two FP16 terms hi + lo (22 significant bits, like the TF32 pairs of
+// a 3xTF32 product; the scaling bounds every entry of L by 2, so the terms' absolute
+// rounding is that of FP32 relative to the row's norm).  Products take three terms
+// (lo hi + hi lo + hi hi; Ootomo and Yokota, "Recovering single precision accuracy from
+// Tensor Cores while surpassing the FP32 theoretical peak performance", IJHPCA 2022) with
+// FP32 accumulation.  The factor only preconditions the double-float refinement.
+//
+// 400 centres, two 8-warp blocks per SM: 195 us against 410 us of a right-looking
+// Cholesky with 3xTF32 products on an FP32 matrix in memory (its tile updates loaded and
+// stored their target and split both operands every time; the same sweeps to converge).
+// The m16n8k16 FP16 MMA issues in 8 cycles, the same as m16n8k8 TF32 at half the depth.
+//
+// A tile is stored in the register layout of the m16n8k16 A operand: 16-byte element
+// (4 t + 2 mt + ks) * 32 + lane (t = 0: hi, 1: lo; mt: 16 rows; ks: 16 columns).  The
+// same registers are the B operand of the transposed tile, so every product is
+// D += X Y^T of two stored tiles, read by 16-byte loads without a conversion.  The
+// diagonal slots hold W_kk = inv(L_kk), so that the columns below a diagonal tile and the
+// substitutions are products too.  Tile (i, j), i >= j, is at 256 (i (i + 1) / 2 + j);
+// until it is final its slot holds the FP32 accumulator of its owner warp, lane by lane.
+constexpr int TILE16 = 256;   // 16-byte elements per tile
+constexpr int WS_LD = 34;     // row stride (floats) of the diagonal tile's staging
+constexpr size_t CHOL_SMEM = (size_t)(32 * WS_LD + 64) * sizeof(float);
+// tiles of subdomains of at most 96 unknowns (6 tiles, 24 KB) stay in shared memory:
+// with the padding to 32 they could exceed the (m + 6)^2 floats of the slot in memory
+constexpr int SMALL_T = 3;
 
-// Tiles of 32 x 32 held in registers, one row per lane (a[c] = element (r, c) of
-// the tile, r = lane); rows/columns beyond m read as the identity.
-__device__ __forceinline__ void tile_load(const float* B, int m, int ld, int ti, int tj,
-                                          float (&a)[32], int lane) {
-  const int r = 32 * ti + lane;
-#pragma unroll
-  for (int c = 0; c < 32; ++c) {
-    const int col = 32 * tj + c;
-    a[c] = (r < m && col < m) ? B[(int64_t)col * ld + r] : ((r == col) ? 1.f : 0.f);
-  }
-}
-__device__ __forceinline__ void tile_store(float* B, int m, int ld, int ti, int tj,
-                                           const float (&a)[32], int lane, bool lower_only) {
-  const int r = 32 * ti + lane;
-  if (r >= m) return;
-#pragma unroll
-  for (int c = 0; c < 32; ++c) {
-    const int col = 32 * tj + c;
-    if (col < m && (!lower_only || c <= lane)) B[(int64_t)col * ld + r] = a[c];
-  }
-}
+__device__ __forceinline__ int tile_at(int i, int j) { return TILE16 * (i * (i + 1) / 2 + j); }
 
-// POTRF of one 32 x 32 tile held in registers (a[c] = element (lane, c)): writes the
-// factor's lower triangle to tile (k, k) of B, its rows (zero right of the diagonal)
-// and 1 / L_jj (column 32) to Lkk; sets *s_flag on a non-positive pivot.
-__device__ __forceinline__ void potrf_tile(float (&a)[32], float* B, int m, int ld, int k,
-                                           float* Lkk, int lane, int* s_flag) {
-  const unsigned full = 0xffffffffu;
-  bool bad = false;
-  float dg = 1.f;
-#pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    float djj = __shfl_sync(full, a[j], j);
-    if (!(djj > 0.f)) {
-      bad = true;
-      djj = 1.f;
-    }
-    const float rs = rsqrtf(djj);  // FP32 factor: refinement absorbs its rounding
-    const float sq = djj * rs;
-    if (lane == j) dg = sq;
-    const float lrj = (lane > j) ? a[j] * rs : ((lane == j) ? sq : 0.f);
-    if (lane >= j) a[j] = lrj;
-    // the row update in chunks of 8 shuffles: the fence keeps the compiler from
-    // hoisting all 31 (the row a[] then stays in registers under the cap)
-#pragma unroll
-    for (int c0 = (j + 1) & ~7; c0 < 32; c0 += 8) {
-#pragma unroll
-      for (int c = c0; c < c0 + 8; ++c) {
-        if (c <= j) continue;
-        const float lcj = __shfl_sync(full, lrj, c);
-        if (lane >= c) a[c] = fmaf(-lrj, lcj, a[c]);
-      }
-      __syncwarp();
-    }
-  }
-  if (bad && lane == 0) *s_flag = 1;
-  tile_store(B, m, ld, k, k, a, lane, true);
-#pragma unroll
-  for (int c = 0; c < 32; ++c) Lkk[lane * TS + c] = (c < lane) ? a[c] : 0.f;
-  Lkk[lane * TS + 32] = 1.f / dg;
-}
-
-// Swizzle of the shared tile column: element (t, r) of a 32 x 32 tile (t the column
-// of L_ik, r its row) sits at t * 32 + (r ^ pswz(t)).  The tensor-core fragments read
-// rows r = 8a + g (g = lane / 4) of columns t = 8b + q (q = lane % 4): the XOR sends
-// the four q to four different groups of eight banks.  An aligned group of four r
-// stays contiguous and in order (float4 reads of a row).
-__device__ __forceinline__ int pswz(int t) { return (t & 3) << 3; }
-
-__device__ __forceinline__ uint32_t to_tf32(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
-}
-// x = hi + lo with hi and lo TF32 (the split of the 3xTF32 products: Ootomo and
-// Yokota, "Recovering single precision accuracy from Tensor Cores while surpassing
-// the FP32 theoretical peak performance", IJHPCA 2022)
-__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
-  hi = to_tf32(x);
-  lo = to_tf32(x - __uint_as_float(hi));
-}
-__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4],
-                                         const uint32_t (&b)[2]) {
+__device__ __forceinline__ void mma_f16(float (&c)[4], const uint4& a, uint32_t b0, uint32_t b1) {
   asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
       "{%8,%9}, {%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+      : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
 }
 
-// Tile (i, j) of B -= L_ik L_jk^T on the tensor cores (warp-level m16n8k8 TF32 MMA),
-// FP32-accurate by the 3xTF32 split (hi*hi + hi*lo + lo*hi, FP32 accumulation): the
-// factor only preconditions the double-float refinement, which absorbs the ~2^-21
-// relative rounding like the FP32 one.  The 32 x 32 tile is 2 x 4 fragments of
-// 16 x 8; Pi, Pj: the swizzled shared tiles of L_ik and L_jk.  Entries past m are
-// neither read nor written; a diagonal tile keeps its upper triangle.
-__device__ __forceinline__ void tile_update_mma(float* B, int m, int ld, int ti, int tj,
-                                                const float* Pi, const float* Pj, int lane) {
-  const int g = lane >> 2, q = lane & 3;
-  float c[2][4][4];
+// (x, y) = hi + lo as two packed FP16 pairs
+__device__ __forceinline__ void split_f16(float x, float y, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(x, y);
+  const float2 hf = __half22float2(h);
+  const __half2 l = __floats2half2_rn(x - hf.x, y - hf.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// transpose of an 8 x 8 block of 16-bit elements held one row pair per lane
+__device__ __forceinline__ uint32_t trans8(uint32_t v) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
+
+// a stored tile in registers: u[t][mt][ks]
+struct Tile16 {
+  uint4 u[2][2][2];
+  __device__ __forceinline__ void load(const uint4* p, int lane) {
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
+    for (int s = 0; s < 8; ++s) u[s >> 2][(s >> 1) & 1][s & 1] = p[32 * s + lane];
+  }
+  __device__ __forceinline__ void store(uint4* p, int lane) const {
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int r = 32 * ti + 16 * mt + g + 8 * (e >> 1);
-        const int col = 32 * tj + 8 * nt + 2 * q + (e & 1);
-        c[mt][nt][e] = (r < m && col < m) ? B[(int64_t)col * ld + r] : 0.f;
-      }
-#pragma unroll
-  for (int ks = 0; ks < 4; ++ks) {
-    const int t0 = 8 * ks + q, t1 = t0 + 4;  // both have (t & 3) == q
-    const int sw = q << 3;
-    uint32_t ah[2][4], al[2][4], bh[4][2], bl[4][2];
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt) {
-      const int r0 = (16 * mt + g) ^ sw, r1 = (16 * mt + g + 8) ^ sw;
-      split_tf32(-Pi[t0 * 32 + r0], ah[mt][0], al[mt][0]);
-      split_tf32(-Pi[t0 * 32 + r1], ah[mt][1], al[mt][1]);
-      split_tf32(-Pi[t1 * 32 + r0], ah[mt][2], al[mt][2]);
-      split_tf32(-Pi[t1 * 32 + r1], ah[mt][3], al[mt][3]);
-    }
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      const int rn = (8 * nt + g) ^ sw;
-      split_tf32(Pj[t0 * 32 + rn], bh[nt][0], bl[nt][0]);
-      split_tf32(Pj[t1 * 32 + rn], bh[nt][1], bl[nt][1]);
-    }
+    for (int s = 0; s < 8; ++s) p[32 * s + lane] = u[s >> 2][(s >> 1) & 1][s & 1];
+  }
+  // the tile of the accumulators sign * c (C layout of the m16n8k16 MMA)
+  __device__ __forceinline__ void from_acc(const float (&c)[2][4][4], float sign) {
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        mma_tf32(c[mt][nt], al[mt], bh[nt]);
-        mma_tf32(c[mt][nt], ah[mt], bl[nt]);
-        mma_tf32(c[mt][nt], ah[mt], bh[nt]);
+      for (int ks = 0; ks < 2; ++ks) {
+        const float(&p)[4] = c[mt][2 * ks];
+        const float(&q)[4] = c[mt][2 * ks + 1];
+        uint4 &h = u[0][mt][ks], &l = u[1][mt][ks];
+        split_f16(sign * p[0], sign * p[1], h.x, l.x);
+        split_f16(sign * p[2], sign * p[3], h.y, l.y);
+        split_f16(sign * q[0], sign * q[1], h.z, l.z);
+        split_f16(sign * q[2], sign * q[3], h.w, l.w);
       }
   }
-  const bool diag = ti == tj;
+  // this tile := its transpose
+  __device__ __forceinline__ void transpose() {
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      uint4 v[2][2];
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+          const uint4 s = u[t][ks][mt];
+          v[mt][ks] = make_uint4(trans8(s.x), trans8(s.z), trans8(s.y), trans8(s.w));
+        }
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) u[t][mt][ks] = v[mt][ks];
+    }
+  }
+};
+
+// c += X Y^T, three terms
+__device__ __forceinline__ void tile_mma(float (&c)[2][4][4], const Tile16& X, const Tile16& Y) {
+#pragma unroll
+  for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+    for (int term = 0; term < 3; ++term)  // lo hi, hi lo, hi hi
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          const uint4& y = Y.u[term == 1][nt >> 1][ks];
+          mma_f16(c[mt][nt], X.u[term == 0][mt][ks], (nt & 1) ? y.y : y.x, (nt & 1) ? y.w : y.z);
+        }
+}
+
+// c = -(D B D) tile (i, j) (identity past m), from the high terms of B
+__device__ __forceinline__ void tile_from_B(float (&c)[2][4][4], const float2* __restrict__ B,
+                                            int m, int ld, const float* dsc, int i, int j,
+                                            int lane) {
+  const int g = lane >> 2, q = lane & 3;
 #pragma unroll
   for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int rl = 16 * mt + g + 8 * (e >> 1), cl = 8 * nt + 2 * q + (e & 1);
-        const int r = 32 * ti + rl, col = 32 * tj + cl;
-        if (r < m && col < m && (!diag || cl <= rl)) B[(int64_t)col * ld + r] = c[mt][nt][e];
+        const int r = 32 * i + 16 * mt + g + 8 * (e >> 1);
+        const int col = 32 * j + 8 * nt + 2 * q + (e & 1);
+        float v = (r == col) ? -1.f : 0.f;
+        if (r < m && col < m) v = -B[(int64_t)col * ld + r].x * (dsc[r] * dsc[col]);
+        c[mt][nt][e] = v;
       }
 }
 
-// Shared memory of chol_factor for an m x m matrix: two L_kk tiles (rows of TS
-// floats) and the current tile column, transposed (T - 1 tiles of 32 x 32).
-__host__ __device__ inline size_t chol_scratch_bytes(int m) {
-  const int T = (m + 31) / 32;
-  return (size_t)2 * 32 * TS * sizeof(float) + (size_t)(T > 1 ? T - 1 : 0) * 1024 * sizeof(float);
+// accumulators <-> a tile slot, each lane its own values
+__device__ __forceinline__ void acc_store(uint4* p, const float (&c)[2][4][4], int lane) {
+  float4* f = reinterpret_cast<float4*>(p);
+#pragma unroll
+  for (int s = 0; s < 8; ++s) {
+    const float(&v)[4] = c[s >> 2][s & 3];
+    f[32 * s + lane] = make_float4(v[0], v[1], v[2], v[3]);
+  }
+}
+__device__ __forceinline__ void acc_load(const uint4* p, float (&c)[2][4][4], int lane) {
+  const float4* f = reinterpret_cast<const float4*>(p);
+#pragma unroll
+  for (int s = 0; s < 8; ++s) {
+    const float4 v = f[32 * s + lane];
+    c[s >> 2][s & 3][0] = v.x;
+    c[s >> 2][s & 3][1] = v.y;
+    c[s >> 2][s & 3][2] = v.z;
+    c[s >> 2][s & 3][3] = v.w;
+  }
 }
 
-// Right-looking tiled Cholesky (lower) of the m x m matrix B (column-major, ld), in
-// place (lower triangle).  Per tile column k: warps solve the tiles below the
-// diagonal (one row per lane, rows of L_kk read as float4 broadcasts) and keep them,
-// transposed and swizzled, in shared memory; then they update the trailing tile
-// pairs on the tensor cores (3xTF32 warp MMA, both factors read from the shared tile
-// column: the update loads only its own tile).  Lookahead: warp 0 first updates the next
-// diagonal tile and factorises it in registers (shuffles) while the other warps
-// update the rest; the tiles go to the warps in the order they finish.
-// scratch: chol_scratch_bytes(m), 16-byte aligned.  False on a non-positive pivot.
+// W = inv(L) of the diagonal tile -c = L L^T, by Gauss elimination of [A | I] with one
+// column of both halves per lane: step j publishes row j of A (by symmetry the
+// multipliers of every row) in shared memory, and each lane takes its multiple off its
+// two columns, two rows per packed FMA.  Rows of the eliminated identity over the square
+// roots of the pivots are W, staged and stored as a tile at p.  A chain of 32 steps of
+// one shared-memory round trip and one reciprocal (a Cholesky of the tile, then its
+// inverse, are two chains of shuffles).  Sets *s_flag on a pivot that is not positive.
+__device__ __forceinline__ void diag_inverse(const float (&c)[2][4][4], uint4* p, float* ws,
+                                             int lane, int* s_flag) {
+  const int g = lane >> 2, q = lane & 3;
+  float* s = ws + 32 * WS_LD;  // two rows of 32
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        ws[(16 * mt + g + 8 * (e >> 1)) * WS_LD + 8 * nt + 2 * q + (e & 1)] = -c[mt][nt][e];
+  __syncwarp();
+  float2 a[16], w[16];
+#pragma unroll
+  for (int r = 0; r < 16; ++r) {
+    a[r] = *reinterpret_cast<const float2*>(ws + lane * WS_LD + 2 * r);
+    w[r] = make_float2(2 * r == lane ? 1.f : 0.f, 2 * r + 1 == lane ? 1.f : 0.f);
+  }
+  bool ok = true;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    float* sj = s + 32 * (j & 1);
+    sj[lane] = (j & 1) ? a[j >> 1].y : a[j >> 1].x;
+    __syncwarp();
+    const float d = sj[j];
+    ok &= d > 0.f;
+    const float inv = __fdividef(1.f, d);
+    const float fa = -inv * ((j & 1) ? a[j >> 1].y : a[j >> 1].x);
+    const float wj = (j & 1) ? w[j >> 1].y : w[j >> 1].x;
+    const float fw = -inv * wj;
+    if (!(j & 1)) {
+      const float l = sj[j + 1];
+      a[j >> 1].y = fmaf(l, fa, a[j >> 1].y);
+      w[j >> 1].y = fmaf(l, fw, w[j >> 1].y);
+      w[j >> 1].x = wj * rsqrtf(d);
+    } else {
+      w[j >> 1].y = wj * rsqrtf(d);
+    }
+#pragma unroll
+    for (int r = (j >> 1) + 1; r < 16; ++r) {
+      const float2 l = *reinterpret_cast<const float2*>(sj + 2 * r);
+      a[r] = __ffma2_rn(l, make_float2(fa, fa), a[r]);
+      w[r] = __ffma2_rn(l, make_float2(fw, fw), w[r]);
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < 16; ++r) {
+    ws[(2 * r) * WS_LD + lane] = w[r].x;
+    ws[(2 * r + 1) * WS_LD + lane] = w[r].y;
+  }
+  if (!__all_sync(0xffffffffu, ok) && lane == 0) *s_flag = 1;
+  __syncwarp();
+  Tile16 t;
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks) {
+      uint4 &h = t.u[0][mt][ks], &l = t.u[1][mt][ks];
+      const float* b = ws + (16 * mt + g) * WS_LD + 16 * ks + 2 * q;
+      split_f16(b[0], b[1], h.x, l.x);
+      split_f16(b[8 * WS_LD], b[8 * WS_LD + 1], h.y, l.y);
+      split_f16(b[8], b[9], h.z, l.z);
+      split_f16(b[8 * WS_LD + 8], b[8 * WS_LD + 9], h.w, l.w);
+    }
+  t.store(p, lane);
+  __syncwarp();
+}
+
+// The factor of D B D into the tiles LP.  Phase k makes column k: a row's warp takes the
+// last term off its accumulator, multiplies by W_kk^T, stores L_ik, takes L_ik L_ik^T off
+// its diagonal tile, then accumulates the terms j < k of column k + 1.  Warp 0 has row
+// k + 1 and goes on to the inverse of diagonal tile k + 1, the serial chain of the
+// factorisation, while the other warps do the bulk; one barrier per phase.  Every
+// accumulator stays with the warp that owns its row in that phase.  False on a pivot that
+// is not positive.
 template <int NT>
-__device__ bool chol_factor(float* B, int m, int ld, float* scratch, int* s_flag,
-                            int* s_next) {
+__device__ __noinline__ bool chol_factor(const float2* __restrict__ B, int m, int ld, const float* dsc,
+                            uint4* LP, float* ws, int* s_flag) {
   constexpr int NW = NT / 32;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const unsigned full = 0xffffffffu;
   const int T = (m + 31) / 32;
-  // two L_kk buffers (step k reads buffer k & 1 while step k + 1's is written); row
-  // j: L_kk[j][c] for c < j (0 elsewhere), [32] = 1 / L_jj
-  float* Lkk0 = scratch;
-  // tile column k: tile i > k at P + (i - k - 1) * 1024, element
-  // [t * 32 + (r ^ pswz(t))] = L_ik[r][t]
-  float* P = scratch + 2 * 32 * TS;
-  if (threadIdx.x == 0) *s_flag = 0;
-  __syncthreads();
+  float c[2][4][4];
   if (wid == 0) {
-    float a[32];
-    tile_load(B, m, ld, 0, 0, a, lane);
-    potrf_tile(a, B, m, ld, 0, Lkk0, lane, s_flag);
+    tile_from_B(c, B, m, ld, dsc, 0, 0, lane);
+    diag_inverse(c, LP, ws, lane, s_flag);
   }
   __syncthreads();
-  for (int k = 0; k < T; ++k) {
-    const float* Lkk = Lkk0 + (k & 1) * 32 * TS;
-    // TRSM: tiles (i, k), i > k: X L_kk^T = A_ik, row by row in each lane
-    for (int i = k + 1 + wid; i < T; i += NW) {
-      float b[32];
-      tile_load(B, m, ld, i, k, b, lane);
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        float v = b[j];
-#pragma unroll
-        for (int c4 = 0; c4 < (j + 3) / 4; ++c4) {  // entries c >= j of row j are 0
-          const float4 q = *reinterpret_cast<const float4*>(Lkk + j * TS + 4 * c4);
-          v = fmaf(-b[4 * c4], q.x, v);
-          v = fmaf(-b[4 * c4 + 1], q.y, v);
-          v = fmaf(-b[4 * c4 + 2], q.z, v);
-          v = fmaf(-b[4 * c4 + 3], q.w, v);
-        }
-        b[j] = v * Lkk[j * TS + 32];
-        if ((j & 3) == 3) __syncwarp();  // bounds the broadcasts in flight (registers)
-      }
-      tile_store(B, m, ld, i, k, b, lane, false);
-      float* Pi = P + (i - k - 1) * 1024;
-      const bool rin = 32 * i + lane < m;  // rows past m: zero (their updates are unused)
-#pragma unroll
-      for (int t = 0; t < 32; ++t) Pi[t * 32 + (lane ^ pswz(t))] = rin ? b[t] : 0.f;
-    }
-    if (threadIdx.x == 0) *s_next = NW;
-    __syncthreads();
-    if (k + 1 >= T) break;
-    // trailing update: tiles (i, j), k < j <= i; pair 0 is tile (k + 1, k + 1)
-    const int n = T - k - 1;
-    const int npairs = n * (n + 1) / 2;
-    int pidx = wid;
-    while (pidx < npairs) {
-      int ii = (int)((sqrtf(8.f * pidx + 1.f) - 1.f) * 0.5f);
-      while ((ii + 1) * (ii + 2) / 2 <= pidx) ++ii;
-      while (ii * (ii + 1) / 2 > pidx) --ii;
-      const int jj = pidx - ii * (ii + 1) / 2;
-      const int i = k + 1 + ii, j = k + 1 + jj;
-      const float* Pi = P + ii * 1024;
-      const float* Pj = P + jj * 1024;
-      if (pidx == 0) {
-        // the next diagonal tile in row layout (one row per lane) for its
-        // factorisation: acc -= L_ik L_jk^T with L_ik[lane][t] and the row t of L_jk^T
-        // from shared memory, packed FP32x2 FMAs
-        float acc[32];
-        tile_load(B, m, ld, i, j, acc, lane);
-#pragma unroll 4
-        for (int t = 0; t < 32; ++t) {
-          const int sw = pswz(t);
-          const float l = -Pi[t * 32 + (lane ^ sw)];
-          const float2 lr = make_float2(l, l);
-#pragma unroll
-          for (int c4 = 0; c4 < 8; ++c4) {
-            const float4 q = *reinterpret_cast<const float4*>(Pj + t * 32 + ((4 * c4) ^ sw));
-            float2 a01 = make_float2(acc[4 * c4], acc[4 * c4 + 1]);
-            float2 a23 = make_float2(acc[4 * c4 + 2], acc[4 * c4 + 3]);
-            a01 = __ffma2_rn(lr, make_float2(q.x, q.y), a01);
-            a23 = __ffma2_rn(lr, make_float2(q.z, q.w), a23);
-            acc[4 * c4] = a01.x;
-            acc[4 * c4 + 1] = a01.y;
-            acc[4 * c4 + 2] = a23.x;
-            acc[4 * c4 + 3] = a23.y;
-          }
-        }
-        potrf_tile(acc, B, m, ld, k + 1, Lkk0 + ((k + 1) & 1) * 32 * TS, lane, s_flag);
+  for (int k = 0; k + 1 < T; ++k) {
+    for (int i = k + 1 + wid; i < T; i += (wid == 0) ? T : NW - 1) {
+      Tile16 X, Y;
+      uint4* slot = LP + tile_at(i, k);
+      if (k == 0) {
+        tile_from_B(c, B, m, ld, dsc, i, 0, lane);
       } else {
-        tile_update_mma(B, m, ld, i, j, Pi, Pj, lane);
+        acc_load(slot, c, lane);
+        X.load(LP + tile_at(i, k - 1), lane);
+        Y.load(LP + tile_at(k, k - 1), lane);
+        tile_mma(c, X, Y);
       }
-      int nxt = 0;
-      if (lane == 0) nxt = atomicAdd(s_next, 1);
-      pidx = __shfl_sync(full, nxt, 0);
+      X.from_acc(c, -1.f);
+      Y.load(LP + tile_at(k, k), lane);
+#pragma unroll
+      for (int e = 0; e < 32; ++e) c[e >> 4][(e >> 2) & 3][e & 3] = 0.f;
+      tile_mma(c, X, Y);
+      X.from_acc(c, 1.f);
+      X.store(slot, lane);
+      uint4* dslot = LP + tile_at(i, i);
+      if (k == 0)
+        tile_from_B(c, B, m, ld, dsc, i, i, lane);
+      else
+        acc_load(dslot, c, lane);
+      tile_mma(c, X, X);
+      if (i == k + 1) {
+        diag_inverse(c, dslot, ws, lane, s_flag);
+      } else {
+        acc_store(dslot, c, lane);
+        // column k + 1 of this row, terms j < k
+        tile_from_B(c, B, m, ld, dsc, i, k + 1, lane);
+        for (int j = 0; j < k; ++j) {
+          X.load(LP + tile_at(i, j), lane);
+          Y.load(LP + tile_at(k + 1, j), lane);
+          tile_mma(c, X, Y);
+        }
+        acc_store(LP + tile_at(i, k + 1), c, lane);
+      }
     }
     __syncthreads();
   }
   return *s_flag == 0;
 }
 
-// Inverses of the diagonal tiles of the factor L (lower, column-major, ld), for
-// chol_solve2: tile k's inverse (lower triangular) packed by columns at dinv + 528 k,
-// column c holding rows c..31 from tri_colstart(c).  Reading row i (fixed column,
-// consecutive rows) or column c (rows i >= c: offsets that are triangular numbers
-// apart, distinct modulo 32) is free of bank conflicts.  Rows and columns past m are
-// the identity's.
-__device__ __forceinline__ int tri_colstart(int c) { return 32 * c - (c * (c - 1)) / 2; }
-constexpr int TRI_TILE = 528;  // 32 * 33 / 2
-
-template <int NT>
-__device__ void chol_diag_inverses(const float* __restrict__ L, int m, int ld, float* dinv) {
-  constexpr int NW = NT / 32;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const unsigned full = 0xffffffffu;
-  const int T = (m + 31) / 32;
-  for (int k = wid; k < T; k += NW) {
-    float a[32];  // a[j] = L[32 k + lane][32 k + j] (only j <= lane is read below)
-    tile_load(L, m, ld, k, k, a, lane);
-    float dl = 1.f;  // L[lane][lane] (constant indices keep a[] in registers)
+// The B operand (K = 32, N = 8) holding the two right-hand sides of block k in its first
+// two columns (zeros in the others): b[t][ks] = (b0, b1).
+__device__ __forceinline__ void rhs_frags(const float* rx, const float* ry, int lane,
+                                          uint2 (&b)[2][2]) {
+  const int g = lane >> 2, q = lane & 3;
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (j == lane) dl = a[j];
-    const float rdiag = 1.f / dl;
-    // lane i: row i of X = inv(L_kk), right-looking: row j is final once scaled by
-    // 1 / L_jj, then every later row i takes off L_ij X_j (independent columns: the
-    // dependent chain is 32 steps long, not 528)
-    float x[32];
-#pragma unroll
-    for (int c = 0; c < 32; ++c) x[c] = (c == lane) ? 1.f : 0.f;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const float rj = __shfl_sync(full, rdiag, j);
-#pragma unroll
-      for (int c = 0; c <= j; ++c) {
-        const float xjc = __shfl_sync(full, x[c], j) * rj;
-        if (lane == j)
-          x[c] = xjc;
-        else if (lane > j)
-          x[c] = fmaf(-a[j], xjc, x[c]);
-      }
+  for (int ks = 0; ks < 2; ++ks) {
+    b[0][ks] = b[1][ks] = make_uint2(0u, 0u);
+    if (g < 2) {
+      const float* v = (g ? ry : rx) + 16 * ks + 2 * q;
+      const float2 v0 = *reinterpret_cast<const float2*>(v);
+      const float2 v1 = *reinterpret_cast<const float2*>(v + 8);
+      split_f16(v0.x, v0.y, b[0][ks].x, b[1][ks].x);
+      split_f16(v1.x, v1.y, b[0][ks].y, b[1][ks].y);
     }
-    float* D = dinv + TRI_TILE * k + lane;
-#pragma unroll
-    for (int c = 0; c < 32; ++c)
-      if (c <= lane) D[tri_colstart(c) - c] = x[c];
   }
-  __syncthreads();
 }
 
-// Solve (L L^T) x = r in place for two right-hand sides (float).  L: lower m x m,
-// column-major, leading dimension ld (a multiple of 4, 16-byte aligned base); only
-// its lower triangle is read.  rx, ry: shared, 16-byte aligned, zero from m up to a
-// multiple of 32.  dinv: the diagonal tiles' inverses (chol_diag_inverses), so that
-// a diagonal step is a triangular product in one warp instead of a chain of 32
-// dependent shuffles.  By tiles of 32: the off-diagonal tiles by all warps with
-// coalesced (forward) or contiguous float4 (backward) loads, issued before the
-// barrier that publishes the diagonal step (their values do not depend on it), and
-// float4 broadcasts of x.  part: 64 * warps floats.
-template <int NT>
-__device__ void chol_solve2(const float* __restrict__ L, int m, int ld, float* rx, float* ry,
-                            float* part, const float* dinv) {
-  constexpr int NW = NT / 32;
+// d[mt] = rows 16 mt + g and + 8 of X v (columns 2 q, 2 q + 1: the right-hand sides are
+// in the lanes q = 0); the three terms in accumulators of their own (chains of two MMAs)
+__device__ __forceinline__ void tile_vec(float (&d)[2][4], const Tile16& X,
+                                         const uint2 (&b)[2][2]) {
+  float t[3][2][4];
+#pragma unroll
+  for (int e = 0; e < 24; ++e) t[e >> 3][(e >> 2) & 1][e & 3] = 0.f;
+#pragma unroll
+  for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+    for (int term = 0; term < 3; ++term)
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt) {
+        const uint2& v = b[term == 1][ks];
+        mma_f16(t[term][mt], X.u[term == 0][mt][ks], v.x, v.y);
+      }
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) d[mt][e] = (t[0][mt][e] + t[1][mt][e]) + t[2][mt][e];
+}
+
+__device__ __forceinline__ void cp_async16(void* smem, const void* g) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(smem)),
+               "l"(g)
+               : "memory");
+}
+
+// rows of block n of the right-hand sides: minus d, or d
+__device__ __forceinline__ void rhs_put(float* rx, float* ry, const float (&d)[2][4],
+                                        bool subtract, int lane) {
+  if ((lane & 3) == 0) {
+    float* x = rx + (lane >> 2);
+    float* y = ry + (lane >> 2);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {  // rows g + 8 h
+      const float vx = d[h >> 1][2 * (h & 1)], vy = d[h >> 1][2 * (h & 1) + 1];
+      x[8 * h] = subtract ? x[8 * h] - vx : vx;
+      y[8 * h] = subtract ? y[8 * h] - vy : vy;
+    }
+  }
+  __syncwarp();
+}
+
+// Block substitution over the tiles: forward (L y = r) or backward (L^T x = y).  Warp 0
+// runs the serial chain: it takes block n - 1's solution off block n and multiplies by
+// the inverse of the diagonal tile; its two tiles per step come through a ring of three
+// stages in shared memory (asynchronous copies, each lane its own elements).  After the
+// barrier that publishes block k's solution the other warps take it off blocks k + 2 and
+// on (each block with its warp), their next tile loaded a step ahead.  One barrier per
+// step.  ring: null when the tiles are in shared memory themselves.
+constexpr int RING_STAGES = 3;
+constexpr size_t RING_BYTES = (size_t)RING_STAGES * 2 * TILE16 * sizeof(uint4);
+template <int NT, bool BACK>
+__device__ __noinline__ void tri_solve(const uint4* LP, int T, float* rx, float* ry,
+                                       uint4* ring) {
+  constexpr int NO = NT / 32 - 1;  // warps beside the chain's
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // blocks in the order of the substitution: n-th block
+  auto blk = [&](int n) { return BACK ? T - 1 - n : n; };
+  auto tile_of = [&](int n, int k) {  // the tile coupling block n to block k (k before n)
+    return BACK ? tile_at(blk(k), blk(n)) : tile_at(blk(n), blk(k));
+  };
+  uint2 b[2][2];
+  float d[2][4];
+  if (wid == 0) {
+    auto issue = [&](int n) {
+      if (ring != nullptr && n < T) {
+        uint4* dst = ring + (n % RING_STAGES) * 2 * TILE16;
+        const uint4* w = LP + tile_at(blk(n), blk(n));
+#pragma unroll
+        for (int e = 0; e < 8; ++e) cp_async16(dst + 32 * e + lane, w + 32 * e + lane);
+        if (n > 0) {
+          const uint4* x = LP + tile_of(n, n - 1);
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            cp_async16(dst + TILE16 + 32 * e + lane, x + 32 * e + lane);
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    issue(0);
+    issue(1);
+    for (int n = 0; n < T; ++n) {
+      issue(n + 2);
+      asm volatile("cp.async.wait_group %0;" ::"n"(RING_STAGES - 1) : "memory");
+      const uint4* src = ring + (n % RING_STAGES) * 2 * TILE16;
+      Tile16 X, W;
+      W.load(ring != nullptr ? src : LP + tile_at(blk(n), blk(n)), lane);
+      if (BACK) W.transpose();
+      float* bx = rx + 32 * blk(n);
+      float* by = ry + 32 * blk(n);
+      if (n > 0) {
+        X.load(ring != nullptr ? src + TILE16 : LP + tile_of(n, n - 1), lane);
+        if (BACK) X.transpose();
+        __syncthreads();  // block n - 1 is published, the earlier ones are off block n
+        tile_vec(d, X, b);
+        rhs_put(bx, by, d, true, lane);
+      }
+      rhs_frags(bx, by, lane, b);
+      tile_vec(d, W, b);
+      __syncwarp();
+      rhs_put(bx, by, d, false, lane);
+      rhs_frags(bx, by, lane, b);
+    }
+    __syncthreads();
+  } else {
+    // this warp's first block from block n on
+    auto first_of = [&](int n) { return n + (wid - 1 - n % NO + NO) % NO; };
+    Tile16 X, N;
+    int n0 = first_of(2);
+    if (n0 < T) X.load(LP + tile_of(n0, 0), lane);
+    for (int k = 0; k < T; ++k) {
+      const int n1 = first_of(k + 3);
+      if (n1 < T) N.load(LP + tile_of(n1, k + 1), lane);
+      if (BACK) X.transpose();
+      __syncthreads();  // block k is published
+      if (n0 < T) {
+        rhs_frags(rx + 32 * blk(k), ry + 32 * blk(k), lane, b);
+        tile_vec(d, X, b);
+        rhs_put(rx + 32 * blk(n0), ry + 32 * blk(n0), d, true, lane);
+        for (int n = n0 + NO; n < T; n += NO) {
+          X.load(LP + tile_of(n, k), lane);
+          if (BACK) X.transpose();
+          tile_vec(d, X, b);
+          rhs_put(rx + 32 * blk(n), ry + 32 * blk(n), d, true, lane);
+        }
+      }
+      X = N;
+      n0 = n1;
+    }
+  }
+}
+
+// rx, ry := D (L L^T)^-1 D of them, two right-hand sides (shared, 16-byte aligned, zero
+// from m up to a multiple of 32), each scaled by a power of two to a largest value in
+// [1, 2) for the FP16 terms.
+template <int NT>
+__device__ void chol_solve2(const uint4* LP, int m, const float* dsc, float* rx, float* ry,
+                            double* sh, uint4* ring) {
   const int T = (m + 31) / 32;
-  // ---- forward: L y = r
-  for (int k = 0; k < T; ++k) {
-    const int r0 = 32 * k;
-    // this warp's first off-diagonal tile (k + 1 + wid), loaded ahead
-    const int ia = k + 1 + wid;
-    const int ra = 32 * ia + lane;
-    float la[32];
-    if (ia < T && ra < m) {
-      const float* Lc = L + (int64_t)r0 * ld + ra;
-#pragma unroll
-      for (int c = 0; c < 32; ++c) la[c] = Lc[(int64_t)c * ld];
-    }
-    if (wid == 0) {
-      // y_k = inv(L_kk) r_k: lane i sums row i of the inverse
-      const float* D = dinv + TRI_TILE * k + lane;
-      float vx = 0.f, vy = 0.f;
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        if (j <= lane) {
-          const float l = D[tri_colstart(j) - j];
-          vx = fmaf(l, rx[r0 + j], vx);
-          vy = fmaf(l, ry[r0 + j], vy);
-        }
-      }
-      __syncwarp();
-      rx[r0 + lane] = vx;
-      ry[r0 + lane] = vy;
-    }
-    __syncthreads();
-    // r_i -= L_ik y_k for the tiles i > k (their rows are below m only in full tiles k)
-    for (int i = ia; i < T; i += NW) {
-      const int r = 32 * i + lane;
-      if (r < m) {
-        if (i != ia) {
-          const float* Lc = L + (int64_t)r0 * ld + r;
-#pragma unroll
-          for (int c = 0; c < 32; ++c) la[c] = Lc[(int64_t)c * ld];
-        }
-        float sx = 0.f, sy = 0.f, sx2 = 0.f, sy2 = 0.f;
-#pragma unroll
-        for (int c4 = 0; c4 < 8; c4 += 2) {
-          const float4 yx = *reinterpret_cast<const float4*>(rx + r0 + 4 * c4);
-          const float4 yy = *reinterpret_cast<const float4*>(ry + r0 + 4 * c4);
-          const float4 yx2 = *reinterpret_cast<const float4*>(rx + r0 + 4 * c4 + 4);
-          const float4 yy2 = *reinterpret_cast<const float4*>(ry + r0 + 4 * c4 + 4);
-          sx = fmaf(la[4 * c4], yx.x, sx);
-          sy = fmaf(la[4 * c4], yy.x, sy);
-          sx = fmaf(la[4 * c4 + 1], yx.y, sx);
-          sy = fmaf(la[4 * c4 + 1], yy.y, sy);
-          sx = fmaf(la[4 * c4 + 2], yx.z, sx);
-          sy = fmaf(la[4 * c4 + 2], yy.z, sy);
-          sx = fmaf(la[4 * c4 + 3], yx.w, sx);
-          sy = fmaf(la[4 * c4 + 3], yy.w, sy);
-          sx2 = fmaf(la[4 * c4 + 4], yx2.x, sx2);
-          sy2 = fmaf(la[4 * c4 + 4], yy2.x, sy2);
-          sx2 = fmaf(la[4 * c4 + 5], yx2.y, sx2);
-          sy2 = fmaf(la[4 * c4 + 5], yy2.y, sy2);
-          sx2 = fmaf(la[4 * c4 + 6], yx2.z, sx2);
-          sy2 = fmaf(la[4 * c4 + 6], yy2.z, sy2);
-          sx2 = fmaf(la[4 * c4 + 7], yx2.w, sx2);
-          sy2 = fmaf(la[4 * c4 + 7], yy2.w, sy2);
-        }
-        rx[r] -= sx + sx2;
-        ry[r] -= sy + sy2;
-      }
-    }
-    __syncthreads();
+  float mx = 0.f, my = 0.f;
+  for (int i = threadIdx.x; i < m; i += NT) {
+    rx[i] *= dsc[i];
+    ry[i] *= dsc[i];
+    mx = fmaxf(mx, fabsf(rx[i]));
+    my = fmaxf(my, fabsf(ry[i]));
   }
-  // ---- backward: L^T x = y
-  for (int k = T - 1; k >= 0; --k) {
-    const int c0 = 32 * k;
-    const int t = c0 + lane;  // this lane's column
-    float px = 0.f, py = 0.f;
-    for (int i = k + 1 + wid; i < T; i += NW) {  // column t is below m here
-      const float* Lc = L + (int64_t)t * ld + 32 * i;
-      float4 lv[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int row = 32 * i + 4 * q;
-        lv[q] = (row < ld) ? *reinterpret_cast<const float4*>(Lc + 4 * q)
-                           : make_float4(0.f, 0.f, 0.f, 0.f);
-        if (row + 0 >= m) lv[q].x = 0.f;
-        if (row + 1 >= m) lv[q].y = 0.f;
-        if (row + 2 >= m) lv[q].z = 0.f;
-        if (row + 3 >= m) lv[q].w = 0.f;
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int row = 32 * i + 4 * q;
-        const float4 xv = *reinterpret_cast<const float4*>(rx + row);
-        const float4 yv = *reinterpret_cast<const float4*>(ry + row);
-        px = fmaf(lv[q].x, xv.x, px);
-        py = fmaf(lv[q].x, yv.x, py);
-        px = fmaf(lv[q].y, xv.y, px);
-        py = fmaf(lv[q].y, yv.y, py);
-        px = fmaf(lv[q].z, xv.z, px);
-        py = fmaf(lv[q].z, yv.z, py);
-        px = fmaf(lv[q].w, xv.w, px);
-        py = fmaf(lv[q].w, yv.w, py);
-      }
-    }
-    part[wid * 64 + lane] = px;
-    part[wid * 64 + 32 + lane] = py;
-    __syncthreads();
-    if (wid == 0) {
-      float vx = rx[t], vy = ry[t];
-#pragma unroll
-      for (int w = 0; w < NW; ++w) {
-        vx -= part[w * 64 + lane];
-        vy -= part[w * 64 + 32 + lane];
-      }
-      rx[t] = vx;
-      ry[t] = vy;
-      __syncwarp();
-      // x_k = inv(L_kk)^T v_k: lane c sums column c of the inverse (rows i >= c)
-      const float* D = dinv + TRI_TILE * k + tri_colstart(lane) - lane;
-      float sx = 0.f, sy = 0.f;
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        if (i >= lane) {
-          const float l = D[i];
-          sx = fmaf(l, rx[c0 + i], sx);
-          sy = fmaf(l, ry[c0 + i], sy);
-        }
-      }
-      __syncwarp();
-      rx[t] = sx;
-      ry[t] = sy;
-    }
-    __syncthreads();
+  const float2 mxy = block_max2<NT>(mx, my, sh);
+  const int ex = mxy.x > 0.f && mxy.x < INFINITY ? ilogbf(mxy.x) : 0;
+  const int ey = mxy.y > 0.f && mxy.y < INFINITY ? ilogbf(mxy.y) : 0;
+  for (int i = threadIdx.x; i < m; i += NT) {
+    rx[i] = ldexpf(rx[i], -ex);
+    ry[i] = ldexpf(ry[i], -ey);
   }
+  __syncthreads();
+  tri_solve<NT, false>(LP, T, rx, ry, ring);
+  tri_solve<NT, true>(LP, T, rx, ry, ring);
+  for (int i = threadIdx.x; i < m; i += NT) {
+    rx[i] = ldexpf(rx[i] * dsc[i], ex);
+    ry[i] = ldexpf(ry[i] * dsc[i], ey);
+  }
+  __syncthreads();
 }
 
 // Shared-memory layout of k_tps_solve_mp for subdomains of at most n centres.
@@ -741,7 +757,7 @@ struct MpLayout {
   size_t f2_off; // float2: zx, zy, gx, gy (np each)
   size_t f_off;  // float: vx, vy, rx, ry (np each)
   size_t i2_off; // int2: lattice coordinates (np)
-  size_t p_off;  // panel: (2 + warps) * 32 * TS floats at least
+  size_t p_off;  // panel: panel_bytes(warps)
   size_t bytes;
   __host__ __device__ MpLayout(int n, int warps) {
     np = (n + 31) & ~31;
@@ -750,16 +766,7 @@ struct MpLayout {
     f_off = f2_off + (size_t)4 * np * sizeof(float2);
     i2_off = f_off + (size_t)4 * np * sizeof(float);
     p_off = i2_off + (size_t)np * sizeof(int2);
-    // the panel also holds the projection's per-warp tiles and the solves' partial
-    // sums; the Cholesky scratch starts at f2_off (the f2, f and i2 regions are free
-    // while it runs)
-    size_t pbytes = (size_t)(2 + warps) * 32 * TS * sizeof(float);
-    // the solves: per-warp partial sums, then the diagonal tiles' inverses
-    const size_t sol = ((size_t)64 * warps + (size_t)((n + 31) / 32) * TRI_TILE) * sizeof(float);
-    if (pbytes < sol) pbytes = sol;
-    const size_t chol = chol_scratch_bytes(n);
-    if (f2_off + chol > p_off + pbytes) pbytes = f2_off + chol - p_off;
-    bytes = p_off + pbytes;
+    bytes = p_off + panel_bytes(warps);
   }
 };
 
@@ -768,8 +775,8 @@ struct MpLayout {
 //
 // Buffers per subdomain (offset mat_off, a multiple of 4 elements): matrices holds
 // B22 = (Q^T A Q)[3:, 3:] as (hi, lo) float pairs, both triangles, leading
-// dimension mp = m rounded up to 4; matrices32 holds its FP32 Cholesky factor (lower
-// triangle, same layout).
+// dimension mp = m rounded up to 4; matrices32 holds the tiles of its Cholesky factor
+// (chol_factor; in shared memory for small subdomains).
 template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT)
     k_tps_solve_mp(const fi_tps_plan* plan_ptr, const double* cx, const double* cy,
@@ -784,11 +791,12 @@ __global__ void __launch_bounds__(NT, 512 / NT)
                    const int32_t* order, int max_refine, int n_layout) {
   constexpr int NW = NT / 32;
   extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ double sh[80];
-  __shared__ double s_tau[3];
+  __shared__ double sh[BLOCK_SUMS];
+  __shared__ double s_sum[16];
+  __shared__ double s_tau[3], s_T[9];
   __shared__ double s_R[9];
-  __shared__ double s_q1[6];
-  __shared__ int s_flag, s_next, s_bad[2], s_lat;
+  __shared__ double s_q1[6], s_c[6], s_a[6];
+  __shared__ int s_flag, s_bad[2], s_lat;
   const fi_tps_plan p = *plan_ptr;
   // a cluster of csize CTAs per subdomain (1 without cluster launch): all of them
   // factor P and share the FP64 build and projection, rank 0 then solves alone
@@ -829,7 +837,6 @@ __global__ void __launch_bounds__(NT, 512 / NT)
 
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   float2* B2 = reinterpret_cast<float2*>(matrices + mat_off[sd]);
-  float* L32 = matrices32 + mat_off[sd];
 
   if (threadIdx.x == 0)
     s_lat = (cxy2 != nullptr && c_on_lattice != nullptr && phi_table != nullptr) ? *c_on_lattice : 0;
@@ -942,62 +949,79 @@ __global__ void __launch_bounds__(NT, 512 / NT)
     }
   };
 
-  // ---- Householder QR of P = [1, y, x] (FP64), V rows k hold v_k (zeros above k)
+  // ---- Householder QR of P = [1, y, x] (FP64), V rows k hold v_k (zeros above k).  The
+  // first reflector follows from N alone; each of the others needs one block-wide sum
+  // (its norm, with its product with the next column); thread 0 does the scalar FP64 work.
   {
-    double* P0 = W;  // scratch columns
-    double* P1 = W + n;
-    double* P2 = W + 2 * n;
+    double* Va = V;
+    double* Vb = V + n;
+    double* Vc = V + 2 * n;
+    double s2[2] = {0.0, 0.0};
     for (int i = threadIdx.x; i < N; i += NT) {
-      P0[i] = 1.0;
-      P1[i] = yc[i];
-      P2[i] = xc[i];
+      s2[0] += yc[i];
+      s2[1] += xc[i];
+    }
+    block_sums<NT, 2>(s2, sh, s_sum);
+    if (threadIdx.x == 0) {
+      const double rn = sqrt((double)N), tau = 1.0 / ((double)N + rn);
+      s_tau[0] = tau;
+      s_R[0] = -rn;
+      s_c[0] = tau * (s_sum[0] + rn * yc[0]);
+      s_c[1] = tau * (s_sum[1] + rn * xc[0]);
+      s_c[2] = 1.0 + rn;
+      s_flag = 0;
     }
     __syncthreads();
-    double* cols[3] = {P0, P1, P2};
-    bool rank_ok = true;
-    for (int k = 0; k < 3; ++k) {
-      double* x = cols[k];
-      double nrm2 = 0.0;
-      for (int i = k + threadIdx.x; i < N; i += NT) nrm2 += x[i] * x[i];
-      nrm2 = bsum<NT>(nrm2, sh);
-      const double x0 = x[k];
-      const double nrm = sqrt(nrm2);
-      if (!(nrm > 0.0)) {
-        rank_ok = false;
-        break;
+    s2[0] = s2[1] = 0.0;
+    for (int i = threadIdx.x; i < N; i += NT) {
+      const double v = (i == 0) ? s_c[2] : 1.0;
+      const double y = yc[i] - s_c[0] * v, x = xc[i] - s_c[1] * v;
+      Va[i] = v;
+      if (i == 0) {
+        s_R[1] = y;
+        s_R[2] = x;
+        Vb[0] = Vc[0] = 0.0;
+      } else {
+        Vb[i] = y;
+        Vc[i] = x;
+        s2[0] += y * y;
+        s2[1] += y * x;
       }
-      const double alpha = (x0 >= 0.0) ? -nrm : nrm;
-      double* v = V + (int64_t)k * n;
-      for (int i = threadIdx.x; i < N; i += NT) v[i] = (i < k) ? 0.0 : x[i];
-      __syncthreads();
-      if (threadIdx.x == 0) v[k] = x0 - alpha;
-      __syncthreads();
-      double vv = 0.0;
-      for (int i = k + threadIdx.x; i < N; i += NT) vv += v[i] * v[i];
-      vv = bsum<NT>(vv, sh);
-      if (!(vv > 0.0)) {
-        rank_ok = false;
-        break;
-      }
-      const double tau = 2.0 / vv;
-      if (threadIdx.x == 0) {
-        s_tau[k] = tau;
-        s_R[k * 3 + k] = alpha;
-      }
-      for (int j = k + 1; j < 3; ++j) {  // apply H_k to the remaining columns
-        double* y = cols[j];
-        double d = 0.0;
-        for (int i = k + threadIdx.x; i < N; i += NT) d += v[i] * y[i];
-        d = bsum<NT>(d, sh);
-        for (int i = k + threadIdx.x; i < N; i += NT) y[i] -= tau * d * v[i];
-        __syncthreads();
-        if (threadIdx.x == 0) s_R[k * 3 + j] = y[k];
-        __syncthreads();
-      }
-      if (fabs(alpha) < 1e-9 * sqrt((double)N)) rank_ok = false;  // collinear centres
+    }
+    block_sums<NT, 2>(s2, sh, s_sum);
+    const double tiny = 1e-9 * 1e-9 * (double)N;  // collinear centres: |R_kk|^2 below it
+    if (threadIdx.x == 0) {
+      const double q = s_sum[0], y1 = Vb[1];
+      if (!(q >= tiny)) s_flag = 1;
+      const double alpha = (y1 >= 0.0) ? -sqrt(q) : sqrt(q);
+      s_tau[1] = 1.0 / (q - alpha * y1);  // 2 / |v|^2, |v|^2 = 2 (q - alpha y1)
+      s_R[4] = alpha;
+      s_c[0] = s_tau[1] * (s_sum[1] - alpha * Vc[1]);
+      Vb[1] = y1 - alpha;
     }
     __syncthreads();
-    if (!rank_ok) return;
+    double s1[1] = {0.0};
+    for (int i = 1 + threadIdx.x; i < N; i += NT) {
+      const double x = Vc[i] - s_c[0] * Vb[i];
+      if (i == 1) {
+        s_R[5] = x;
+        Vc[1] = 0.0;
+      } else {
+        Vc[i] = x;
+        s1[0] += x * x;
+      }
+    }
+    block_sums<NT, 1>(s1, sh, s_sum);
+    if (threadIdx.x == 0) {
+      const double q = s_sum[0], x2 = Vc[2];
+      if (!(q >= tiny)) s_flag = 1;
+      const double alpha = (x2 >= 0.0) ? -sqrt(q) : sqrt(q);
+      s_tau[2] = 1.0 / (q - alpha * x2);
+      s_R[8] = alpha;
+      Vc[2] = x2 - alpha;
+    }
+    __syncthreads();
+    if (s_flag != 0) return;
   }
   const double* V0 = V;
   const double* V1 = V + n;
@@ -1046,7 +1070,7 @@ __global__ void __launch_bounds__(NT, 512 / NT)
         b = t;
       }
       rs = NW / a;  // nloc * rs is a multiple of NW
-      const int max_jobs = (int)((size_t)(2 + NW) * 32 * TS * sizeof(float) / (96 * sizeof(float2)));
+      const int max_jobs = (int)(panel_bytes(NW) / (96 * sizeof(float2)));
       while (rs > 1 && (nloc * rs > max_jobs || 8 * rs > N)) rs >>= 1;
     }
     float2* part = reinterpret_cast<float2*>(panel);  // [job][3][32]
@@ -1109,23 +1133,22 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   double* Z1 = W + n;
   double* Z2 = W + 2 * n;
   {
-    __shared__ double s_T[9], s_M[9];
+    __shared__ double s_M[9];
     const double* Vk[3] = {V0, V1, V2};
     const double* Yk[3] = {Y0, Y1, Y2};
-    double vtv[3], vty[9];
-    for (int a = 0; a < 3; ++a) {
-      vtv[a] = 0.0;
-      for (int b = 0; b < 3; ++b) vty[3 * a + b] = 0.0;
-    }
+    double pr[12];  // V^T V above the diagonal, V^T Y
+    for (int a = 0; a < 12; ++a) pr[a] = 0.0;
     for (int i = threadIdx.x; i < N; i += NT) {
-      vtv[0] += V0[i] * V1[i];
-      vtv[1] += V0[i] * V2[i];
-      vtv[2] += V1[i] * V2[i];
+      pr[0] += V0[i] * V1[i];
+      pr[1] += V0[i] * V2[i];
+      pr[2] += V1[i] * V2[i];
+#pragma unroll
       for (int a = 0; a < 3; ++a)
-        for (int b = 0; b < 3; ++b) vty[3 * a + b] += Vk[a][i] * Yk[b][i];
+#pragma unroll
+        for (int b = 0; b < 3; ++b) pr[3 + 3 * a + b] += Vk[a][i] * Yk[b][i];
     }
-    for (int a = 0; a < 3; ++a) vtv[a] = bsum<NT>(vtv[a], sh);
-    for (int a = 0; a < 9; ++a) vty[a] = bsum<NT>(vty[a], sh);
+    block_sums<NT, 12>(pr, sh, s_sum);
+    const double *vtv = s_sum, *vty = s_sum + 3;
     if (threadIdx.x == 0) {
       double T[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
       T[0] = s_tau[0];
@@ -1240,13 +1263,11 @@ __global__ void __launch_bounds__(NT, 512 / NT)
               if (in0) {
                 const float2 sv = make_float2(hi.x, lo.x);
                 __stcs(B2 + (int64_t)c * mp + r, sv);  // streaming: keeps L2 for the factor
-                L32[(int64_t)c * mp + r] = sv.x;
                 S[(qb + u) * 33 + lane] = sv;
               }
               if (in1) {
                 const float2 sv = make_float2(hi.y, lo.y);
                 __stcs(B2 + (int64_t)(c + 1) * mp + r, sv);
-                L32[(int64_t)(c + 1) * mp + r] = sv.x;
                 S[(qb + u + 1) * 33 + lane] = sv;
               }
             }
@@ -1265,18 +1286,23 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   }
   cluster.sync();  // the cluster's B tiles are in global memory, visible to rank 0
   if (crank != 0) return;
-  // ---- FP32 Cholesky of B22
-  if (!chol_factor<NT>(L32, m, mp, reinterpret_cast<float*>(smraw + lay.f2_off), &s_flag,
-                       &s_next))
-    return;
-
-  // the diagonal tiles' inverses, after the per-warp partial sums of the solves
-  float* dinv = panel + 64 * NW;
-  chol_diag_inverses<NT>(L32, m, mp, dinv);
+  // ---- Cholesky factor of D B22 D (D in xc: the centres are no longer needed)
+  float* dsc = reinterpret_cast<float*>(xc);
+  if (threadIdx.x == 0) s_flag = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < m; i += NT) {
+    const float v = B2[(int64_t)i * mp + i].x;
+    if (!(v > 0.f)) s_flag = 1;
+    dsc[i] = (v > 0.f) ? ldexpf(1.f, -(ilogbf(v) >> 1)) : 1.f;
+  }
+  __syncthreads();
+  uint4* LP = (m <= 32 * SMALL_T)
+                  ? reinterpret_cast<uint4*>(smraw + lay.p_off + ((CHOL_SMEM + 15) & ~(size_t)15))
+                  : reinterpret_cast<uint4*>(matrices32 + mat_off[sd]);
+  if (!chol_factor<NT>(B2, m, mp, dsc, LP, panel, &s_flag)) return;
+  uint4* ring = (m <= 32 * SMALL_T) ? nullptr : reinterpret_cast<uint4*>(panel);
 
   // ---- outlier iterations with refined solves (x and y in lockstep)
-  double* tx = W;
-  double* ty = W + n;
   double* wx = W + 2 * n;
   double* wy = W + 3 * n;
   for (int r = threadIdx.x; r < lay.np; r += NT) {
@@ -1292,22 +1318,45 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   bool z_zero = true;
   int nsweeps = 0;
   while (true) {
-    // g = Q^T u: rows 3.. as double-float for the refinement, rows 0..2 for a
-    for (int i = threadIdx.x; i < N; i += NT) {
-      tx[i] = (double)vx[i];
-      ty[i] = (double)vy[i];
+    // g = Q^T u = u - V T^T (V^T u): rows 3.. as double-float for the refinement, rows
+    // 0..2 for a
+    {
+      double pr[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+      for (int i = threadIdx.x; i < N; i += NT) {
+        const double ux_ = (double)vx[i], uy_ = (double)vy[i];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const double v = V[k * n + i];
+          pr[k] = fma(v, ux_, pr[k]);
+          pr[3 + k] = fma(v, uy_, pr[3 + k]);
+        }
+      }
+      block_sums<NT, 6>(pr, sh, s_sum);
+      if (threadIdx.x < 6) {  // T^T (V^T u)
+        const int k = threadIdx.x % 3, o = threadIdx.x - k;
+        double t = 0.0;
+        for (int j = 0; j <= k; ++j) t = fma(s_T[3 * j + k], s_sum[o + j], t);
+        s_c[threadIdx.x] = t;
+      }
+      __syncthreads();
+      for (int i = threadIdx.x; i < N; i += NT) {
+        double gxv = (double)vx[i], gyv = (double)vy[i];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const double v = V[k * n + i];
+          gxv = fma(-v, s_c[k], gxv);
+          gyv = fma(-v, s_c[3 + k], gyv);
+        }
+        if (i < 3) {
+          s_q1[i] = gxv;
+          s_q1[3 + i] = gyv;
+        } else {
+          gx2[i - 3] = df_split(gxv);
+          gy2[i - 3] = df_split(gyv);
+        }
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    apply_reflectors2<NT, false>(V, n, s_tau, N, tx, ty, sh);
-    for (int i = threadIdx.x; i < m; i += NT) {
-      gx2[i] = df_split(tx[i + 3]);
-      gy2[i] = df_split(ty[i + 3]);
-    }
-    if (threadIdx.x < 3) {
-      s_q1[threadIdx.x] = tx[threadIdx.x];
-      s_q1[3 + threadIdx.x] = ty[threadIdx.x];
-    }
-    __syncthreads();
     // refine z (B z = g): FP32 Cholesky solves, double-float residuals
     bool conv = false;
     double prev = INFINITY;
@@ -1322,18 +1371,22 @@ __global__ void __launch_bounds__(NT, 512 / NT)
       } else {
         residual_df2<NT>(B2, m, mp, zx2, zy2, gx2, gy2, rx, ry);
       }
-      chol_solve2<NT>(L32, m, mp, rx, ry, panel, dinv);
+      chol_solve2<NT>(LP, m, dsc, rx, ry, sh, ring);
       ++nsweeps;
-      double dmax = 0.0, zmax = 0.0;
+      float dm = 0.f, zm = 0.f;
       for (int i = threadIdx.x; i < m; i += NT) {
         if (!done[0]) zx2[i] = df_add(zx2[i], make_float2(rx[i], 0.f));
         if (!done[1]) zy2[i] = df_add(zy2[i], make_float2(ry[i], 0.f));
-        dmax = fmax(dmax, fmax(done[0] ? 0.0 : fabs((double)rx[i]),
-                               done[1] ? 0.0 : fabs((double)ry[i])));
-        zmax = fmax(zmax, fmax(fabs((double)zx2[i].x), fabs((double)zy2[i].x)));
+        // (beyond the FP16 range of the factor's products the corrections are not finite:
+        // their bits compare as the largest)
+        const unsigned ax = done[0] ? 0u : __float_as_uint(fabsf(rx[i]));
+        const unsigned ay = done[1] ? 0u : __float_as_uint(fabsf(ry[i]));
+        dm = __uint_as_float(max(__float_as_uint(dm), max(ax, ay)));
+        zm = fmaxf(zm, fmaxf(fabsf(zx2[i].x), fabsf(zy2[i].x)));
       }
-      dmax = bmax<NT>(dmax, sh);
-      zmax = bmax<NT>(zmax, sh);
+      const float2 dz = block_max2<NT>(dm, zm, sh);
+      if (!(dz.x < INFINITY)) break;  // the FP64 LU takes over
+      const double dmax = (double)dz.x, zmax = (double)dz.y;
       if (dmax == 0.0) {
         conv = true;
         break;
@@ -1359,36 +1412,49 @@ __global__ void __launch_bounds__(NT, 512 / NT)
       break;
     }
     // a = R^-1 (Q1^T u - C z) (R upper triangular); w = Q [0; z]
-    double ax3[3], ay3[3];
     {
-      double c6[6] = {0, 0, 0, 0, 0, 0};
+      // C z and V^T [0; z] of both components in one block-wide sum
+      double pr[12];
+      for (int k = 0; k < 12; ++k) pr[k] = 0.0;
       for (int i = threadIdx.x; i < m; i += NT) {
         const double zxv = df_to_double(zx2[i]), zyv = df_to_double(zy2[i]);
+#pragma unroll
         for (int k = 0; k < 3; ++k) {
-          c6[k] = fma(C[k * n + i], zxv, c6[k]);
-          c6[3 + k] = fma(C[k * n + i], zyv, c6[3 + k]);
+          const double cv = C[k * n + i], v = V[k * n + i + 3];
+          pr[k] = fma(cv, zxv, pr[k]);
+          pr[3 + k] = fma(cv, zyv, pr[3 + k]);
+          pr[6 + k] = fma(v, zxv, pr[6 + k]);
+          pr[9 + k] = fma(v, zyv, pr[9 + k]);
         }
       }
-      for (int k = 0; k < 3; ++k) {
-        const double2 s2 = bsum2<NT>(make_double2(c6[k], c6[3 + k]), sh);
-        c6[k] = s2.x;
-        c6[3 + k] = s2.y;
-      }
-      for (int k = 2; k >= 0; --k) {
-        double sxk = s_q1[k] - c6[k], syk = s_q1[3 + k] - c6[3 + k];
-        for (int j = k + 1; j < 3; ++j) {
-          sxk -= s_R[k * 3 + j] * ax3[j];
-          syk -= s_R[k * 3 + j] * ay3[j];
+      block_sums<NT, 12>(pr, sh, s_sum);
+      if (threadIdx.x < 2) {  // back substitution with R, one component per thread
+        const int o = 3 * threadIdx.x;
+        for (int k = 2; k >= 0; --k) {
+          double t = s_q1[o + k] - s_sum[o + k];
+          for (int j = k + 1; j < 3; ++j) t -= s_R[k * 3 + j] * s_a[o + j];
+          s_a[o + k] = t / s_R[k * 3 + k];
         }
-        ax3[k] = sxk / s_R[k * 3 + k];
-        ay3[k] = syk / s_R[k * 3 + k];
-      }
-      for (int i = threadIdx.x; i < N; i += NT) {
-        wx[i] = (i < 3) ? 0.0 : df_to_double(zx2[i - 3]);
-        wy[i] = (i < 3) ? 0.0 : df_to_double(zy2[i - 3]);
+      } else if (threadIdx.x >= 32 && threadIdx.x < 38) {  // T (V^T [0; z])
+        const int t6 = threadIdx.x - 32, k = t6 % 3, o = t6 - k;
+        double t = 0.0;
+        for (int j = k; j < 3; ++j) t = fma(s_T[3 * k + j], s_sum[6 + o + j], t);
+        s_c[t6] = t;
       }
       __syncthreads();
-      apply_reflectors2<NT, true>(V, n, s_tau, N, wx, wy, sh);
+      for (int i = threadIdx.x; i < N; i += NT) {
+        double a = (i < 3) ? 0.0 : df_to_double(zx2[i - 3]);
+        double b = (i < 3) ? 0.0 : df_to_double(zy2[i - 3]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const double v = V[k * n + i];
+          a = fma(-v, s_c[k], a);
+          b = fma(-v, s_c[3 + k], b);
+        }
+        wx[i] = a;
+        wy[i] = b;
+      }
+      __syncthreads();
     }
     // smoothed = u - lam w; outlier test (compute_tps_weights_iter, subdom.py:236-280)
     if (threadIdx.x == 0) s_bad[0] = s_bad[1] = 0;
@@ -1411,8 +1477,10 @@ __global__ void __launch_bounds__(NT, 512 / NT)
         if (use_threshold && dfy > threshold) by++;
       }
     }
-    mxx = bmax<NT>(mxx, sh);
-    mxy = bmax<NT>(mxy, sh);
+    if (count[0] == 1 || count[1] == 1) {  // max_udiff is that of the first solution
+      mxx = block_max_pos<NT>(mxx, sh);
+      mxy = block_max_pos<NT>(mxy, sh);
+    }
     if (bx) atomicAdd(&s_bad[0], bx);
     if (by) atomicAdd(&s_bad[1], by);
     __syncthreads();
@@ -1434,9 +1502,9 @@ __global__ void __launch_bounds__(NT, 512 / NT)
     }
     if (threadIdx.x == 0) {
       if (fin[0])
-        for (int k = 0; k < 3; ++k) wxo[N + k] = ax3[k];
+        for (int k = 0; k < 3; ++k) wxo[N + k] = s_a[k];
       if (fin[1])
-        for (int k = 0; k < 3; ++k) wyo[N + k] = ay3[k];
+        for (int k = 0; k < 3; ++k) wyo[N + k] = s_a[3 + k];
     }
     // replace the erratic values (rounded to float32 like upstream's array)
     for (int r = threadIdx.x; r < N; r += NT) {

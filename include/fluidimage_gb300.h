@@ -502,8 +502,8 @@ int fi_tps_phi_table2(float* table2, int64_t count, void* stream);
 /*
  * Mixed-precision TPS solve (same inputs and outputs as fi_tps_solve): null-space
  * form B z = Q2^T u with B = Q2^T (K + lam I) Q2 (P = Q R, Householder; B projected
- * in double-float with the compact WY form of Q), factorised in FP32 (blocked Cholesky) and
- * refined with double-float (pairs of floats) residuals g - B z; the affine part is
+ * in double-float with the compact WY form of Q), factorised by a tiled Cholesky on the
+ * tensor cores (FP16 pairs, FP32 accumulation) and refined with double-float (pairs of floats) residuals g - B z; the affine part is
  * a = R^-1 (Q1^T u - Q1^T A Q2 z).  K comes from the phi table.  The outlier
  * iterations of compute_tps_weights_iter (thin_plate_spline_subdom.py:236-280)
  * warm-start from the previous solution.  mat_offsets[i] must be multiples of 4 and
