@@ -156,6 +156,14 @@ _SIGNATURES = {
         [P, P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int,
          C.c_double, P, P],
     ),
+    "fi_rank_subtract": (
+        C.c_int,
+        [P, P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int,
+         C.c_double, C.c_double, C.c_int, C.c_int, P, P],
+    ),
+    "fi_rank_needs_scratch": (C.c_int, [C.c_int] * 7),
+    "fi_sharpen": (C.c_int, [P, P, P, C.c_int, C.c_int, C.c_int, C.c_int, P, C.c_int, P, C.c_int,
+                             C.c_double, P]),
     "fi_subtract_weighted": (
         C.c_int, [P, P, C.c_int, C.c_int64, C.c_double, C.c_int, C.c_int, P, P]),
     "fi_clamp": (C.c_int, [P, C.c_int, C.c_int64, C.c_double, C.c_double, P, P]),

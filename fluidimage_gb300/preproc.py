@@ -148,27 +148,35 @@ def _rank(size, rank_kind, percentile=None):
     return size - 1 if p == 100.0 else int(float(size) * p / 100.0)
 
 
-def rank_filter(img, window, rank_kind, percentile=None, mode="reflect", cval=0.0):
-    """scipy.ndimage minimum_filter / median_filter / percentile_filter of a stack
-    (nt, ny, nx) over the box ``window`` = (st, sy, sx); output in the input dtype."""
+def _rank_args(img, window, rank_kind, percentile, mode, cval):
+    """The checked arguments of a rank filter of a stack (nt, ny, nx) over the box
+    ``window`` = (st, sy, sx): the contiguous stack, its dtype, and what the library's
+    entry points take after the two image pointers, with their scratch (kept until the
+    call)."""
     torch = _torch()
-    lib = L.load()
     x = img.contiguous()
     nt, ny, nx = x.shape
     st, sy, sx = (int(w) for w in window)
     r = _rank(st * sy * sx, rank_kind, percentile)
     if mode not in L.MODES:
         raise RuntimeError(f"boundary mode not supported: {mode}")
-    dt = _DT[_dtype_of(x)]
+    dtype = _dtype_of(x)
+    dt = _DT[dtype]
     if dt in (L.PRE_F32, L.PRE_F64) and bool(torch.isnan(x).any()):
         raise ValueError("rank filters of images with NaN are not provided")
-    out = torch.empty_like(x)
     scratch = None
-    if r in (0, st * sy * sx - 1):
+    if L.load().fi_rank_needs_scratch(dt, nt, ny, st, sy, sx, r):
         scratch = torch.empty(2 * x.numel(), dtype=torch.int64, device=x.device)
-    L.check(lib.fi_rank_filter(L.ptr(x), L.ptr(out), dt, nt, ny, nx, st, sy, sx, r,
-                               L.MODES[mode], float(cval), L.ptr(scratch), L.stream_handle()),
-            "fi_rank_filter")
+    return x, dtype, (dt, nt, ny, nx, st, sy, sx, r, L.MODES[mode], float(cval)), scratch
+
+
+def rank_filter(img, window, rank_kind, percentile=None, mode="reflect", cval=0.0):
+    """scipy.ndimage minimum_filter / median_filter / percentile_filter of a stack
+    (nt, ny, nx) over the box ``window`` = (st, sy, sx); output in the input dtype."""
+    x, _, args, scratch = _rank_args(img, window, rank_kind, percentile, mode, cval)
+    out = _torch().empty_like(x)
+    L.check(L.load().fi_rank_filter(L.ptr(x), L.ptr(out), *args, L.ptr(scratch),
+                                    L.stream_handle()), "fi_rank_filter")
     return out
 
 
@@ -178,16 +186,17 @@ def _result_dtype(dtype, weight):
     return (z - weight * z).dtype
 
 
-def _subtract(img, filtered, weight, clamp):
-    lib = L.load()
-    dtype = _dtype_of(img)
+def _rank_subtract(img, window, rank_kind, percentile, weight, clamp, mode="reflect"):
+    """``img - weight * rank_filter(img, ...)`` in numpy's result dtype (negatives set to
+    0 with ``clamp``), in one pass."""
+    x, dtype, args, scratch = _rank_args(img, window, rank_kind, percentile, mode, 0.0)
     out_dt = _result_dtype(dtype, weight)
     if out_dt not in _DT:
         raise TypeError(f"result dtype {out_dt} not supported")
-    out = _empty(tuple(img.shape), out_dt, img.device)
-    L.check(lib.fi_subtract_weighted(L.ptr(img), L.ptr(filtered), _DT[dtype], img.numel(),
-                                     float(weight), _DT[out_dt], int(clamp), L.ptr(out),
-                                     L.stream_handle()), "fi_subtract_weighted")
+    out = _empty(tuple(x.shape), out_dt, x.device)
+    L.check(L.load().fi_rank_subtract(L.ptr(x), L.ptr(out), *args, float(weight), _DT[out_dt],
+                                      int(clamp), L.ptr(scratch), L.stream_handle()),
+            "fi_rank_subtract")
     return out
 
 
@@ -201,8 +210,8 @@ def _window2d(window_size):
 
 def _sliding(img, weight, window_size, boundary_condition, kind, percentile=None):
     x, single = _stack(img)
-    f = rank_filter(x, _window2d(window_size), kind, percentile, mode=boundary_condition)
-    out = _subtract(x, f, weight, clamp=True)
+    out = _rank_subtract(x, _window2d(window_size), kind, percentile, weight, True,
+                         mode=boundary_condition)
     return out[0] if single else out
 
 
@@ -246,8 +255,7 @@ def _calcul_windowshape(arr_shape, window_shape):
 
 def _temporal(img, weight, window_shape, kind, percentile=None):
     window = _calcul_windowshape(tuple(img.shape), window_shape)
-    f = rank_filter(img, window, kind, percentile)
-    return _subtract(img, f, weight, clamp=False)
+    return _rank_subtract(img, window, kind, percentile, weight, False)
 
 
 def temporal_minima(img, weight=1.0, window_shape=None):
@@ -494,14 +502,31 @@ def adaptive_threshold(img, window_size=5, offset=0):
     return out - offset
 
 
+#: largest filter radius of fi_sharpen
+SHARPEN_MAX_RADIUS = 32
+
+
 @_per_image
 def sharpen(img, sigma1=3.0, sigma2=1.0, alpha=30.0):
     """_toolbox_py.py:472-490: two chained gaussian filters in the image dtype, then
     ``blurred + alpha * (blurred - filter_blurred)`` with numpy's promotions (integer
     images: the difference wraps in their type, the result is float64)."""
+    dtype = _dtype_of(img)
+    if dtype.kind == "u":
+        x, single = _stack(img)
+        x = x.contiguous()
+        nt, ny, nx = x.shape
+        w1, r1 = _gauss_weights(sigma1)
+        w2, r2 = _gauss_weights(sigma2)
+        if max(r1, r2) <= SHARPEN_MAX_RADIUS and nt <= 65535:
+            blurred = _torch().empty_like(x)
+            out = _empty((nt, ny, nx), np.float64, x.device)
+            L.check(L.load().fi_sharpen(L.ptr(x), L.ptr(out), L.ptr(blurred), _DT[dtype], nt, ny,
+                                        nx, w1.ctypes.data, r1, w2.ctypes.data, r2, float(alpha),
+                                        L.stream_handle()), "fi_sharpen")
+            return out[0] if single else out
     blurred = gaussian_filter(img, sigma1)
     filtered = gaussian_filter(blurred, sigma2)
-    dtype = _dtype_of(blurred)
     out_dt = np.dtype(np.float32) if dtype == np.float32 else np.dtype(np.float64)
     out = _empty(tuple(blurred.shape), out_dt, blurred.device)
     L.check(L.load().fi_sharpen_combine(L.ptr(blurred), L.ptr(filtered), _DT[dtype],

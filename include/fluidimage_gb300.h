@@ -622,7 +622,8 @@ int fi_tps_interpolate(const fi_tps_plan* plan, int nb_subdom, int max_members,
  * window st x sy x sx, output in the input dtype: the rank-th smallest window value
  * (scipy.ndimage.rank_filter semantics: window [i - s//2, i - s//2 + s - 1], the
  * boundary mode and cval); rank 0 / st*sy*sx - 1 are the minimum / maximum filters
- * (separable; scratch: 2 * nt*ny*nx uint64), other ranks an exact radix select.
+ * (scratch: 2 * nt*ny*nx uint64 when fi_rank_needs_scratch, else nullable), other
+ * ranks an exact radix select.
  * Replaces ndi.minimum_filter / median_filter / percentile_filter in sliding_* and
  * temporal_* (works/preproc/_toolbox_py.py:66-155, 189-256).
  */
@@ -637,6 +638,17 @@ int fi_rank_filter(const void* in, void* out, int dtype, int nt, int ny, int nx,
  */
 int fi_subtract_weighted(const void* img, const void* filtered, int dtype, int64_t count,
                          double weight, int out_dtype, int clamp, void* out, void* stream);
+
+/*
+ * The rank filter and the subtraction in one pass: out = in - weight * filtered with
+ * the arguments of fi_rank_filter and fi_subtract_weighted (out is not in).
+ */
+int fi_rank_subtract(const void* in, void* out, int dtype, int nt, int ny, int nx, int st, int sy,
+                     int sx, int rank, int mode, double cval, double weight, int out_dtype,
+                     int clamp, void* scratch, void* stream);
+
+/* 1 when fi_rank_filter / fi_rank_subtract need their scratch for this window, else 0. */
+int fi_rank_needs_scratch(int dtype, int nt, int ny, int st, int sy, int sx, int rank);
 
 /* global_threshold (_toolbox_py.py:265-289): values below lo set to lo, above hi to hi. */
 int fi_clamp(const void* in, int dtype, int64_t count, double lo, double hi, void* out,
@@ -741,6 +753,16 @@ int fi_rank_equalize(const uint8_t* in, int ny, int nx, int radius, uint8_t* out
  */
 int fi_gaussian_filter(const void* in, void* out, void* tmp, int dtype, int nt, int ny, int nx,
                        const double* weights, int radius, void* stream);
+
+/*
+ * sharpen of 8 and 16 bit images (_toolbox_py.py:472-490): the gaussian filter with
+ * weights1 into blurred, the one with weights2 on it, and the combination of
+ * fi_sharpen_combine into out (float64).  The weights (2 radius + 1 doubles each,
+ * radius at most 32) are host memory, read before the call returns.
+ */
+int fi_sharpen(const void* in, void* out, void* blurred, int dtype, int nt, int ny, int nx,
+               const double* weights1, int radius1, const double* weights2, int radius2,
+               double alpha, void* stream);
 
 /*
  * sharpen's last line (_toolbox_py.py:489): out = blurred + alpha * (blurred -
