@@ -38,24 +38,44 @@ __device__ __forceinline__ void df_mac(float2 b, float2 z, float& sh, float& sl)
   sh = t;
 }
 
-__device__ __forceinline__ float2 df_neg2(float2 a) { return make_float2(-a.x, -a.y); }
+// a - b of two pairs (an exact product by -1 in a fused multiply-add: one packed
+// instruction, where the negation of a pair would take its own)
+__device__ __forceinline__ float2 df_sub2(float2 a, float2 b) {
+  return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
+}
 
 // Two independent df_mac in the lanes of float2 pairs, with packed FP32x2
 // instructions (each lane rounds exactly as df_mac):
 // (sh.x, sl.x) += b * (zh.x + zl.x) and (sh.y, sl.y) += b * (zh.y + zl.y).
 __device__ __forceinline__ void df_mac_x2(float2 b, float2 zh, float2 zl, float2& sh,
                                           float2& sl) {
-  const float2 bh = make_float2(b.x, b.x), bl = make_float2(b.y, b.y);
+  const float2 bh = make_float2(b.x, b.x), nbh = make_float2(-b.x, -b.x);
+  const float2 nbl = make_float2(-b.y, -b.y);
   const float2 p = __fmul2_rn(bh, zh);
-  float2 e = __ffma2_rn(bh, zh, df_neg2(p));
-  e = __ffma2_rn(bh, zl, e);
-  e = __ffma2_rn(bl, zh, e);
+  float2 ne = __ffma2_rn(nbh, zh, p);  // minus the error of the product
+  ne = __ffma2_rn(nbh, zl, ne);
+  ne = __ffma2_rn(nbl, zh, ne);
   const float2 t = __fadd2_rn(sh, p);
-  const float2 bb = __fadd2_rn(t, df_neg2(sh));
-  const float2 err = __fadd2_rn(__fadd2_rn(sh, df_neg2(__fadd2_rn(t, df_neg2(bb)))),
-                                __fadd2_rn(p, df_neg2(bb)));
-  sl = __fadd2_rn(sl, __fadd2_rn(err, e));
+  const float2 bb = df_sub2(t, sh);
+  const float2 err = __fadd2_rn(df_sub2(sh, df_sub2(t, bb)), df_sub2(p, bb));
+  sl = __fadd2_rn(sl, df_sub2(err, ne));
   sh = t;
+}
+
+// (sh, sl) += (ah, al) in both lanes
+__device__ __forceinline__ void df_acc_x2(float2 ah, float2 al, float2& sh, float2& sl) {
+  const float2 t = __fadd2_rn(sh, ah);
+  const float2 bb = df_sub2(t, sh);
+  const float2 err = __fadd2_rn(df_sub2(sh, df_sub2(t, bb)), df_sub2(ah, bb));
+  sl = __fadd2_rn(sl, __fadd2_rn(err, al));
+  sh = t;
+}
+
+// renormalised: (sh, sl) with sl below half an ulp of sh
+__device__ __forceinline__ void df_norm_x2(float2& sh, float2& sl) {
+  const float2 hi = __fadd2_rn(sh, sl);
+  sl = df_sub2(sl, df_sub2(hi, sh));
+  sh = hi;
 }
 
 }  // namespace fi

@@ -157,119 +157,324 @@ __device__ __forceinline__ double block_max_pos(double v, double* sh) {
   return v;
 }
 
-// bytes of a block's panel: the chunk sums of Y, the projection's per-warp tiles, then
-// the factorisation's staging and the tiles of small subdomains
+// Bytes of a block's panel: the warps' sums of Y with the table of kernel values behind
+// them, then the factorisation's staging with the tiles of small subdomains, then the
+// right-hand sides of the substitutions or the tile products of the residual.
 __host__ __device__ constexpr size_t panel_bytes(int warps) { return (size_t)(2 + warps) * 4608; }
-
-// Start moving [p, p + bytes) from memory into L2 without waiting for it (bulk
-// prefetch by the copy engine; p 16-byte aligned, bytes a multiple of 16).
-__device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+// entries of the table of kernel values
+__host__ __device__ constexpr int panel_table(int warps) {
+  return (int)((panel_bytes(warps) - (size_t)warps * 96 * sizeof(float2)) / sizeof(float2));
 }
 
-// rho = g - B z for two right-hand sides, in double-float; B (m x m, symmetric, both
-// triangles, column-major, leading dimension ld, a multiple of 4; 32-byte aligned)
-// holds (hi, lo) pairs, read with the streaming hint (B is twice the FP32 factor,
-// which should stay in L2).  Each warp takes four columns at a time (one row per
-// lane), then reduce-scatters its eight sums over the warp.  B is streamed from
-// memory: each warp has the copy engine prefetch its next two column groups into L2
-// (contiguous, 32 ld bytes per column) while it works on the current one, so that
-// its loads wait on L2 rather than on memory.  rho is rounded to float.
+// ---- B = Q2^T (K + lam I) Q2 in memory
+// (hi, lo) pairs.  Subdomains of more than 96 unknowns: the 32 x 32 tiles (i, j), i >= j,
+// of its lower half, 1024 pairs each at i (i + 1) / 2 + j, by columns (rows and columns
+// past m zero, diagonal tiles whole): half the bytes of the whole matrix, which the
+// projection writes and every residual reads.  Smaller ones: the whole matrix by columns
+// (leading dimension ld), since padded tiles could exceed the slot.
+constexpr int SMALL_T = 3;
+
+struct BPairs {
+  float2* p;
+  int m, ld;
+  bool tiles;
+  __device__ __forceinline__ float2* tile(int i, int j) const {
+    return p + (size_t)1024 * (i * (i + 1) / 2 + j);
+  }
+  // entry (r, c), r >= c, both below m
+  __device__ __forceinline__ float2 at(int r, int c) const {
+    if (tiles) return tile(r >> 5, c >> 5)[(c & 31) * 32 + (r & 31)];
+    return p[(int64_t)c * ld + r];
+  }
+};
+
+// Sum over the warp of a pair of double-float values held as (x hi, y hi, x lo, y lo).
+__device__ __forceinline__ void df_xor_add(float4& v, int o) {
+  float4 w;
+  w.x = __shfl_xor_sync(0xffffffffu, v.x, o);
+  w.y = __shfl_xor_sync(0xffffffffu, v.y, o);
+  w.z = __shfl_xor_sync(0xffffffffu, v.z, o);
+  w.w = __shfl_xor_sync(0xffffffffu, v.w, o);
+  float2 h = make_float2(v.x, v.y), l = make_float2(v.z, v.w);
+  df_acc_x2(make_float2(w.x, w.y), make_float2(w.z, w.w), h, l);
+  df_norm_x2(h, l);
+  v = make_float4(h.x, h.y, l.x, l.y);
+}
+
+// rho = g - B z for both components, in double-float (z, g: (x hi, y hi, x lo, y lo) per
+// row, zero past m up to a multiple of 32), rounded to float.  A tile is read once and used
+// for its rows and, by symmetry, for its columns: half a tile (16 columns) at a time, one
+// row per lane from memory, staged in shared memory for the columns (lanes 0..15 the
+// columns with rows 0..15, the others with rows 16..31).  A warp takes whole tile columns
+// (J = w, 2 W - 1 - w, ...: a long one with a short one; SPLIT warps share a column's
+// tiles), so that the column sums stay in registers; the row sums of each tile go to `part`
+// (512 bytes per tile below the diagonal), the column sums behind them, and are added in a
+// fixed order at the end.  stage: 16 * 33 pairs per warp.
+__host__ __device__ inline size_t residual_part_bytes(int T, int split) {
+  return (size_t)512 * (T * (T - 1) / 2 + T * split);
+}
+
 template <int NT>
-__device__ __noinline__ void residual_df2(const float2* __restrict__ B, int m, int ld, const float2* zx,
-                             const float2* zy, const float2* gx, const float2* gy, float* rx,
-                             float* ry) {
-  constexpr int NW = NT / 32;
+__device__ __noinline__ void residual_tiles(const BPairs B, const float4* z, const float4* g,
+                                            float* rx, float* ry, float4* part, float2* stage) {
+  constexpr int NW = NT / 32, SPLIT = NW / 8, COLS = NW / SPLIT;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const unsigned full = 0xffffffffu;
-  auto prefetch_group = [&](int c) {
-    if (lane == 0 && c < m)
-      prefetch_l2(B + (int64_t)c * ld, (unsigned)(min(4, m - c) * ld * sizeof(float2)));
-  };
-  prefetch_group(4 * wid);
-  prefetch_group(4 * wid + 4 * NW);
-  for (int c0 = 4 * wid; c0 < m; c0 += 4 * NW) {
-    prefetch_group(c0 + 8 * NW);
-    // column q: x sums in lane .x, y sums in lane .y of the pairs (packed FP32x2)
-    float2 H[4], Lo[4];
+  const int T = (B.m + 31) / 32;
+  float4* colsum = part + 32 * (T * (T - 1) / 2);
+  float2* S = stage + wid * 16 * 33;
+  const int w = wid / SPLIT, sp = wid % SPLIT;
+  const int cq = lane & 15, hf = lane >> 4;
+  for (int round = 0; round * COLS < T; ++round) {
+    const int J = round * COLS + ((round & 1) ? COLS - 1 - w : w);
+    if (J >= T) continue;
+    // column sums of the lane's column in each half
+    float2 ch[2], cl[2];
+    ch[0] = ch[1] = cl[0] = cl[1] = make_float2(0.f, 0.f);
+    for (int I = J + sp; I < T; I += SPLIT) {
+      const float2* tile = B.tile(I, J);
+      float2 rh = make_float2(0.f, 0.f), rl = rh;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) H[q] = Lo[q] = make_float2(0.f, 0.f);
-    const float2* col = B + (int64_t)c0 * ld;
-    const int nc = min(4, m - c0);
-    // two rows per lane and load (16 bytes: twice the bytes in flight per load); ld
-    // is a multiple of 4, so row r + 1 < ld; the padding rows past m are masked
-#pragma unroll 2
-    for (int r = 2 * lane; r < m; r += 64) {
-      const float4 a = *reinterpret_cast<const float4*>(zx + r);
-      const float4 b = *reinterpret_cast<const float4*>(zy + r);
-      const float2 zh0 = make_float2(a.x, b.x), zl0 = make_float2(a.y, b.y);
-      const float2 zh1 = make_float2(a.z, b.z), zl1 = make_float2(a.w, b.w);
-      const bool two = r + 1 < m;
+      for (int h = 0; h < 2; ++h) {
+        float2 v[16];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (q < nc) v = __ldcs(reinterpret_cast<const float4*>(col + (int64_t)q * ld + r));
-        if (!two) v.z = v.w = 0.f;
-        df_mac_x2(make_float2(v.x, v.y), zh0, zl0, H[q], Lo[q]);
-        df_mac_x2(make_float2(v.z, v.w), zh1, zl1, H[q], Lo[q]);
+        for (int q = 0; q < 16; ++q) v[q] = __ldcs(tile + (16 * h + q) * 32 + lane);
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 16; ++q) S[q * 33 + lane] = v[q];
+        if (I != J) {
+          const float4* zc = z + 32 * J + 16 * h;
+#pragma unroll
+          for (int q = 0; q < 16; ++q) {
+            const float4 f = zc[q];
+            df_mac_x2(v[q], make_float2(f.x, f.y), make_float2(f.z, f.w), rh, rl);
+          }
+        }
+        __syncwarp();
+        const float4* zr = z + 32 * I + 16 * hf;
+        const float2* Sc = S + cq * 33 + 16 * hf;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          const float4 f = zr[k];
+          df_mac_x2(Sc[k], make_float2(f.x, f.y), make_float2(f.z, f.w), ch[h], cl[h]);
+        }
       }
-    }
-    float h[8], l[8];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      h[q] = H[q].x;
-      l[q] = Lo[q].x;
-      h[4 + q] = H[q].y;
-      l[4 + q] = Lo[q].y;
-    }
-    // reduce-scatter: lane ends with value 4 b4 + 2 b3 + b2 (b_k = bit k of lane)
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const bool up = lane & 16;
-      const float sh_ = up ? h[k] : h[k + 4], sl_ = up ? l[k] : l[k + 4];
-      const float2 keep = up ? make_float2(h[k + 4], l[k + 4]) : make_float2(h[k], l[k]);
-      const float2 got = make_float2(__shfl_xor_sync(full, sh_, 16), __shfl_xor_sync(full, sl_, 16));
-      const float2 s = df_add(keep, got);
-      h[k] = s.x;
-      l[k] = s.y;
+      if (I != J) part[32 * (I * (I - 1) / 2 + J) + lane] = make_float4(rh.x, rh.y, rl.x, rl.y);
     }
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const bool up = lane & 8;
-      const float sh_ = up ? h[k] : h[k + 2], sl_ = up ? l[k] : l[k + 2];
-      const float2 keep = up ? make_float2(h[k + 2], l[k + 2]) : make_float2(h[k], l[k]);
-      const float2 got = make_float2(__shfl_xor_sync(full, sh_, 8), __shfl_xor_sync(full, sl_, 8));
-      const float2 s = df_add(keep, got);
-      h[k] = s.x;
-      l[k] = s.y;
-    }
-    {
-      const bool up = lane & 4;
-      const float sh_ = up ? h[0] : h[1], sl_ = up ? l[0] : l[1];
-      const float2 keep = up ? make_float2(h[1], l[1]) : make_float2(h[0], l[0]);
-      const float2 got = make_float2(__shfl_xor_sync(full, sh_, 4), __shfl_xor_sync(full, sl_, 4));
-      const float2 s = df_add(keep, got);
-      h[0] = s.x;
-      l[0] = s.y;
-    }
-#pragma unroll
-    for (int o = 2; o > 0; o >>= 1) {
-      const float2 got = make_float2(__shfl_xor_sync(full, h[0], o), __shfl_xor_sync(full, l[0], o));
-      const float2 s = df_add(make_float2(h[0], l[0]), got);
-      h[0] = s.x;
-      l[0] = s.y;
-    }
-    if ((lane & 3) == 0) {
-      const int idx = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-      const int c = c0 + (idx & 3);
-      if (c < m) {
-        const float2 g = (idx >> 2) ? gy[c] : gx[c];
-        const float2 d = df_add(g, make_float2(-h[0], -l[0]));
-        ((idx >> 2) ? ry : rx)[c] = __fadd_rn(d.x, d.y);
-      }
+    for (int h = 0; h < 2; ++h) {
+      float4 v = make_float4(ch[h].x, ch[h].y, cl[h].x, cl[h].y);
+      df_xor_add(v, 16);
+      if (hf == h) colsum[32 * (SPLIT * J + sp) + lane] = v;
     }
   }
   __syncthreads();
+  for (int i = threadIdx.x; i < B.m; i += NT) {
+    const int I = i >> 5, l = i & 31;
+    const float4 gv = g[i];
+    float2 h = make_float2(-gv.x, -gv.y), lo = make_float2(-gv.z, -gv.w);
+    for (int q = 0; q < SPLIT; ++q) {
+      const float4 f = colsum[32 * (SPLIT * I + q) + l];
+      df_acc_x2(make_float2(f.x, f.y), make_float2(f.z, f.w), h, lo);
+    }
+    for (int J = 0; J < I; ++J) {
+      const float4 f = part[32 * (I * (I - 1) / 2 + J) + l];
+      df_acc_x2(make_float2(f.x, f.y), make_float2(f.z, f.w), h, lo);
+    }
+    rx[i] = -__fadd_rn(h.x, lo.x);
+    ry[i] = -__fadd_rn(h.y, lo.y);
+  }
+  __syncthreads();
+}
+
+// The same for the whole matrix of a small subdomain: a warp per column, rows over the
+// lanes.
+template <int NT>
+__device__ __noinline__ void residual_small(const BPairs B, const float4* z, const float4* g,
+                                            float* rx, float* ry) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (int c = wid; c < B.m; c += NT / 32) {
+    float2 h = make_float2(0.f, 0.f), l = h;
+    for (int r = lane; r < B.m; r += 32) {
+      const float4 f = z[r];
+      df_mac_x2(B.p[(int64_t)c * B.ld + r], make_float2(f.x, f.y), make_float2(f.z, f.w), h, l);
+    }
+    float4 v = make_float4(h.x, h.y, l.x, l.y);
+    for (int o = 16; o > 0; o >>= 1) df_xor_add(v, o);
+    if (lane == 0) {
+      const float4 gv = g[c];
+      float2 sh = make_float2(-gv.x, -gv.y), sl = make_float2(-gv.z, -gv.w);
+      df_acc_x2(make_float2(v.x, v.y), make_float2(v.z, v.w), sh, sl);
+      rx[c] = -__fadd_rn(sh.x, sl.x);
+      ry[c] = -__fadd_rn(sh.y, sl.y);
+    }
+  }
+  __syncthreads();
+}
+
+// ---- entries of K
+// kernel value of a pair of centres by log(), as a (hi, lo) pair
+static __device__ __noinline__ float2 phi_far(double xa, double ya, double xb, double yb,
+                                              const double* table, int64_t tsize) {
+  return df_split(phi_pair(xa, ya, xb, yb, table, tsize));
+}
+
+// How a block finds phi of two centres i, j (K_TABLE: every offset of the centres' grid in
+// shared memory, at |code_y| tw + |code_x| of the difference of their codes; K_GATHER: the
+// lattice table in memory by 4 r^2 of their lattice coordinates; K_DIRECT: log()).
+enum KMode { K_TABLE, K_GATHER, K_DIRECT };
+
+struct KEntries {
+  const int2* code;  // grid codes (K_TABLE) or lattice coordinates (K_GATHER)
+  const float2* tab;
+  int tw;
+  const float2* table2;  // (hi, lo) of phi(k / 4), tsz32 entries
+  int tsz32;
+  const double *xc, *yc;
+  const double* table;
+  int64_t tsize;
+  template <int MODE>
+  __device__ __forceinline__ float2 get(int i, int2 ci, int j) const {
+    if (MODE == K_DIRECT) return phi_far(xc[i], yc[i], xc[j], yc[j], table, tsize);
+    const int2 cj = code[j];
+    const int dx = ci.x - cj.x, dy = ci.y - cj.y;
+    if (MODE == K_TABLE) return tab[abs(dy) * tw + abs(dx)];
+    // 4 r^2 in 32-bit integers: the lattice coordinates are below 2^30 in magnitude, so
+    // their differences fit, and |dx|, |dy| <= 32767 keeps dx^2 + dy^2 below 2^31; farther
+    // pairs (beyond the table anyway) take the direct kernel value
+    const bool near = (unsigned)dx + 32767u <= 65534u && (unsigned)dy + 32767u <= 65534u;
+    const int kq = near ? dy * dy + dx * dx : INT_MAX;
+    if (kq < tsz32) return table2[kq];
+    return phi_far(xc[i], yc[i], xc[j], yc[j], nullptr, 0);
+  }
+};
+
+// Y = (K + lam I) V in double-float, one column of the symmetric K per lane.  A column
+// block at a time, the rows shared by the warps, whose sums are added in a fixed order.
+// V's first column is 1 but for its first entry v00, so that sum takes additions only; the
+// others' products run as packed pairs (vy: (v1 hi, v2 hi, v1 lo, v2 lo) per row).  Column
+// blocks are spread over the cluster's blocks; each value is rounded to double and written
+// into every block's Y (3 rows of n).
+template <int NT, int MODE>
+__device__ __noinline__ void build_y(const KEntries K, const float4* vy, const double* V,
+                                     double v00, double lam, int N, int n, double* Y,
+                                     float2* part) {
+  constexpr int NW = NT / 32;
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int r0 = (N * wid / NW) & ~1, r1 = wid == NW - 1 ? N : (N * (wid + 1) / NW) & ~1;
+  for (int cb = crank; 32 * cb < N; cb += csize) {
+    const int c = min(32 * cb + lane, N - 1);
+    const int2 cc = K.code[c];
+    // sums of column 0 over even and odd rows in the lanes of (ah, al); of columns 1 and 2
+    // in the lanes of (bh, bl)
+    float2 ah = make_float2(0.f, 0.f), al = ah, bh = ah, bl = ah;
+    int r = r0;
+#pragma unroll 4
+    for (; r + 1 < r1; r += 2) {
+      const float2 k0 = K.get<MODE>(c, cc, r), k1 = K.get<MODE>(c, cc, r + 1);
+      const float4 f0 = vy[r], f1 = vy[r + 1];
+      df_acc_x2(make_float2(k0.x, k1.x), make_float2(k0.y, k1.y), ah, al);
+      df_mac_x2(k0, make_float2(f0.x, f0.y), make_float2(f0.z, f0.w), bh, bl);
+      df_mac_x2(k1, make_float2(f1.x, f1.y), make_float2(f1.z, f1.w), bh, bl);
+    }
+    if (r < r1) {
+      const float2 k0 = K.get<MODE>(c, cc, r);
+      const float4 f0 = vy[r];
+      df_acc_x2(make_float2(k0.x, 0.f), make_float2(k0.y, 0.f), ah, al);
+      df_mac_x2(k0, make_float2(f0.x, f0.y), make_float2(f0.z, f0.w), bh, bl);
+    }
+    float2* pw = part + wid * 96 + lane;
+    pw[0] = df_add(make_float2(ah.x, al.x), make_float2(ah.y, al.y));
+    pw[32] = make_float2(bh.x, bl.x);
+    pw[64] = make_float2(bh.y, bl.y);
+    __syncthreads();
+    if (wid < 3 && 32 * cb + lane < N) {  // one column of V per warp
+      const float2* q = part + 32 * wid + lane;
+      float2 sum = q[0];
+      for (int w = 1; w < NW; ++w) sum = df_add(sum, q[96 * w]);
+      // K has a zero diagonal: lam v; row 0 of column 0 counted as 1
+      double y = df_to_double(sum) + lam * V[wid * n + c];
+      if (wid == 0) y += (v00 - 1.0) * df_to_double(K.get<MODE>(c, cc, 0));
+      for (int b = 0; b < csize; ++b) {
+        double* Yb = (b == crank) ? Y : cluster.map_shared_rank(Y, b);
+        Yb[wid * n + c] = y;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// B = K + lam I - Z V^T - V Z^T below row and column 3, in double-float, by 32 x 32 tiles
+// (one row per lane, two columns per packed instruction).  V's first column is 1 there, so
+// its two products are additions.  Entries of K up to ~1e5 cancel to B entries ~1e2-1e4;
+// the ~2^-48 |K| rounding leaves B within ~1e-11 of its FP64 value, the interpolated field
+// within ~1e-9 px.  cols: columns -z0, v1, v2, z1, z2 (np / 2 each) as pairs of
+// neighbouring unknowns (hi, hi, lo, lo).
+template <int NT, int MODE>
+__device__ __noinline__ void build_b(const KEntries K, const float4* cols, int np, float2 lam,
+                                     const BPairs B, int crank, int csize) {
+  constexpr int NW = NT / 32;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int m = B.m, N = m + 3;
+  const int T = (m + 31) / 32;
+  const float4 *nz0 = cols, *v1 = nz0 + np / 2, *v2 = v1 + np / 2, *z1 = v2 + np / 2,
+               *z2 = z1 + np / 2;
+  for (int pidx = crank * NW + wid; pidx < T * (T + 1) / 2; pidx += csize * NW) {
+    int I = (int)((sqrtf(8.f * pidx + 1.f) - 1.f) * 0.5f);
+    while ((I + 1) * (I + 2) / 2 <= pidx) ++I;
+    while (I * (I + 1) / 2 > pidx) --I;
+    const int J = pidx - I * (I + 1) / 2;
+    const int r = 32 * I + lane;
+    const int rc = min(r, m - 1);
+    const int2 cr = K.code[rc + 3];
+    auto row_of = [&](const float4* a) {
+      const float4 f = a[rc >> 1];
+      return (rc & 1) ? make_float2(f.y, f.w) : make_float2(f.x, f.z);
+    };
+    const float2 rz0 = row_of(nz0);
+    float2 rv1 = row_of(v1), rv2 = row_of(v2), rz1 = row_of(z1), rz2 = row_of(z2);
+    rv1 = make_float2(-rv1.x, -rv1.y);
+    rv2 = make_float2(-rv2.x, -rv2.y);
+    rz1 = make_float2(-rz1.x, -rz1.y);
+    rz2 = make_float2(-rz2.x, -rz2.y);
+    float2* tile = B.tile(I, J) + lane;
+#pragma unroll 2
+    for (int u = 0; u < 16; ++u) {
+      const int c = 32 * J + 2 * u, q = c >> 1;
+      float2 h = make_float2(0.f, 0.f), l = h;
+      if (c < m) {  // uniform
+        float2 k0 = K.get<MODE>(rc + 3, cr, c + 3), k1 = K.get<MODE>(rc + 3, cr, min(c + 4, N - 1));
+        if (I == J) {  // K has a zero diagonal
+          if (r == c) k0 = lam;
+          if (r == c + 1) k1 = lam;
+        }
+        h = make_float2(k0.x, k1.x);
+        l = make_float2(k0.y, k1.y);
+        const float4 fz0 = nz0[q], fv1 = v1[q], fz1 = z1[q], fv2 = v2[q], fz2 = z2[q];
+        df_acc_x2(make_float2(fz0.x, fz0.y), make_float2(fz0.z, fz0.w), h, l);
+        df_acc_x2(make_float2(rz0.x, rz0.x), make_float2(rz0.y, rz0.y), h, l);
+        df_mac_x2(rz1, make_float2(fv1.x, fv1.y), make_float2(fv1.z, fv1.w), h, l);
+        df_mac_x2(rv1, make_float2(fz1.x, fz1.y), make_float2(fz1.z, fz1.w), h, l);
+        df_mac_x2(rz2, make_float2(fv2.x, fv2.y), make_float2(fv2.z, fv2.w), h, l);
+        df_mac_x2(rv2, make_float2(fz2.x, fz2.y), make_float2(fz2.z, fz2.w), h, l);
+        df_norm_x2(h, l);
+      }
+      if (B.tiles) {  // padding: zeros
+        __stcs(tile + (2 * u) * 32, r < m ? make_float2(h.x, l.x) : make_float2(0.f, 0.f));
+        __stcs(tile + (2 * u + 1) * 32,
+               r < m && c + 1 < m ? make_float2(h.y, l.y) : make_float2(0.f, 0.f));
+      } else if (r < m) {
+        if (c < m) B.p[(int64_t)c * B.ld + r] = make_float2(h.x, l.x);
+        if (c + 1 < m) B.p[(int64_t)(c + 1) * B.ld + r] = make_float2(h.y, l.y);
+        if (I != J) {
+          if (c < m) B.p[(int64_t)r * B.ld + c] = make_float2(h.x, l.x);
+          if (c + 1 < m) B.p[(int64_t)r * B.ld + c + 1] = make_float2(h.y, l.y);
+        }
+      }
+    }
+  }
 }
 
 // ---- Cholesky preconditioner on the tensor cores ------------------------------------
@@ -296,9 +501,12 @@ __device__ __noinline__ void residual_df2(const float2* __restrict__ B, int m, i
 constexpr int TILE16 = 256;   // 16-byte elements per tile
 constexpr int WS_LD = 34;     // row stride (floats) of the diagonal tile's staging
 constexpr size_t CHOL_SMEM = (size_t)(32 * WS_LD + 64) * sizeof(float);
-// tiles of subdomains of at most 96 unknowns (6 tiles, 24 KB) stay in shared memory:
-// with the padding to 32 they could exceed the (m + 6)^2 floats of the slot in memory
-constexpr int SMALL_T = 3;
+// (the tiles of subdomains of at most 32 SMALL_T unknowns, 24 KB, stay in shared memory:
+// with the padding to 32 they could exceed the (m + 6)^2 floats of the slot in memory)
+
+constexpr size_t HV_OFF = 32 * 1024;  // in the panel
+static_assert(CHOL_SMEM + 16 + 6 * TILE16 * sizeof(uint4) <= HV_OFF &&
+                  HV_OFF + 26 * 128 * sizeof(__half) <= panel_bytes(8), "panel");
 
 __device__ __forceinline__ int tile_at(int i, int j) { return TILE16 * (i * (i + 1) / 2 + j); }
 
@@ -388,22 +596,37 @@ __device__ __forceinline__ void tile_mma(float (&c)[2][4][4], const Tile16& X, c
 }
 
 // c = -(D B D) tile (i, j) (identity past m), from the high terms of B
-__device__ __forceinline__ void tile_from_B(float (&c)[2][4][4], const float2* __restrict__ B,
-                                            int m, int ld, const float* dsc, int i, int j,
-                                            int lane) {
+__device__ __forceinline__ void tile_from_B(float (&c)[2][4][4], const BPairs& B,
+                                            const float* dsc, int i, int j, int lane) {
   const int g = lane >> 2, q = lane & 3;
+  const int ld = B.tiles ? 32 : B.ld;
+  const float2* p = (B.tiles ? B.tile(i, j) : B.p + (int64_t)(32 * j) * ld + 32 * i) + 2 * q * ld + g;
+  const int rows = B.m - 32 * i - g, cols = B.m - 32 * j - 2 * q;  // left from this lane's first
+  float dr[4], dc[8];
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
+  for (int a = 0; a < 4; ++a) dr[a] = 8 * a < rows ? dsc[32 * i + g + 8 * a] : 0.f;
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
+  for (int b = 0; b < 8; ++b) {
+    const int cl = 8 * (b >> 1) + (b & 1);
+    dc[b] = cl < cols ? dsc[32 * j + 2 * q + cl] : 0.f;
+  }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int r = 32 * i + 16 * mt + g + 8 * (e >> 1);
-        const int col = 32 * j + 8 * nt + 2 * q + (e & 1);
-        float v = (r == col) ? -1.f : 0.f;
-        if (r < m && col < m) v = -B[(int64_t)col * ld + r].x * (dsc[r] * dsc[col]);
-        c[mt][nt][e] = v;
-      }
+  for (int b = 0; b < 8; ++b)
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const int cl = 8 * (b >> 1) + (b & 1);
+      const bool in = 8 * a < rows && cl < cols;
+      c[a >> 1][b >> 1][2 * (a & 1) + (b & 1)] = in ? p[cl * ld + 8 * a].x : 0.f;
+    }
+#pragma unroll
+  for (int b = 0; b < 8; ++b)
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      float& v = c[a >> 1][b >> 1][2 * (a & 1) + (b & 1)];
+      v *= -dr[a] * dc[b];
+      // the identity past m
+      if (i == j && 8 * a >= rows && g + 8 * a == 2 * q + 8 * (b >> 1) + (b & 1)) v = -1.f;
+    }
 }
 
 // accumulators <-> a tile slot, each lane its own values
@@ -511,14 +734,14 @@ __device__ __forceinline__ void diag_inverse(const float (&c)[2][4][4], uint4* p
 // accumulator stays with the warp that owns its row in that phase.  False on a pivot that
 // is not positive.
 template <int NT>
-__device__ __noinline__ bool chol_factor(const float2* __restrict__ B, int m, int ld, const float* dsc,
-                            uint4* LP, float* ws, int* s_flag) {
+__device__ __noinline__ bool chol_factor(const BPairs B, const float* dsc, uint4* LP, float* ws,
+                                         int* s_flag) {
   constexpr int NW = NT / 32;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int T = (m + 31) / 32;
+  const int T = (B.m + 31) / 32;
   float c[2][4][4];
   if (wid == 0) {
-    tile_from_B(c, B, m, ld, dsc, 0, 0, lane);
+    tile_from_B(c, B, dsc, 0, 0, lane);
     diag_inverse(c, LP, ws, lane, s_flag);
   }
   __syncthreads();
@@ -527,7 +750,7 @@ __device__ __noinline__ bool chol_factor(const float2* __restrict__ B, int m, in
       Tile16 X, Y;
       uint4* slot = LP + tile_at(i, k);
       if (k == 0) {
-        tile_from_B(c, B, m, ld, dsc, i, 0, lane);
+        tile_from_B(c, B, dsc, i, 0, lane);
       } else {
         acc_load(slot, c, lane);
         X.load(LP + tile_at(i, k - 1), lane);
@@ -543,7 +766,7 @@ __device__ __noinline__ bool chol_factor(const float2* __restrict__ B, int m, in
       X.store(slot, lane);
       uint4* dslot = LP + tile_at(i, i);
       if (k == 0)
-        tile_from_B(c, B, m, ld, dsc, i, i, lane);
+        tile_from_B(c, B, dsc, i, i, lane);
       else
         acc_load(dslot, c, lane);
       tile_mma(c, X, X);
@@ -552,7 +775,7 @@ __device__ __noinline__ bool chol_factor(const float2* __restrict__ B, int m, in
       } else {
         acc_store(dslot, c, lane);
         // column k + 1 of this row, terms j < k
-        tile_from_B(c, B, m, ld, dsc, i, k + 1, lane);
+        tile_from_B(c, B, dsc, i, k + 1, lane);
         for (int j = 0; j < k; ++j) {
           X.load(LP + tile_at(i, j), lane);
           Y.load(LP + tile_at(k + 1, j), lane);
@@ -566,26 +789,24 @@ __device__ __noinline__ bool chol_factor(const float2* __restrict__ B, int m, in
   return *s_flag == 0;
 }
 
-// The B operand (K = 32, N = 8) holding the two right-hand sides of block k in its first
-// two columns (zeros in the others): b[t][ks] = (b0, b1).
-__device__ __forceinline__ void rhs_frags(const float* rx, const float* ry, int lane,
-                                          uint2 (&b)[2][2]) {
+// The right-hand sides of the products: 32 rows of the two components as FP16 terms, block
+// k at 128 k: (x hi, x lo, y hi, y lo), 32 each.
+// The B operand (K = 32, N = 8) with the two components in its first two columns (zeros in
+// the others): b[t][ks] = (b0, b1).
+__device__ __forceinline__ void rhs_frags(const __half* hv, int k, int lane, uint2 (&b)[2][2]) {
   const int g = lane >> 2, q = lane & 3;
+  const uint32_t* v = reinterpret_cast<const uint32_t*>(hv + 128 * k + 64 * (g & 1)) + q;
 #pragma unroll
-  for (int ks = 0; ks < 2; ++ks) {
-    b[0][ks] = b[1][ks] = make_uint2(0u, 0u);
-    if (g < 2) {
-      const float* v = (g ? ry : rx) + 16 * ks + 2 * q;
-      const float2 v0 = *reinterpret_cast<const float2*>(v);
-      const float2 v1 = *reinterpret_cast<const float2*>(v + 8);
-      split_f16(v0.x, v0.y, b[0][ks].x, b[1][ks].x);
-      split_f16(v1.x, v1.y, b[0][ks].y, b[1][ks].y);
+  for (int t = 0; t < 2; ++t)
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks) {
+      const uint2 w = make_uint2(v[16 * t + 8 * ks], v[16 * t + 8 * ks + 4]);
+      b[t][ks] = g < 2 ? w : make_uint2(0u, 0u);
     }
-  }
 }
 
-// d[mt] = rows 16 mt + g and + 8 of X v (columns 2 q, 2 q + 1: the right-hand sides are
-// in the lanes q = 0); the three terms in accumulators of their own (chains of two MMAs)
+// d[mt] = rows 16 mt + g and + 8 of X v (columns 2 q, 2 q + 1: the components are in the
+// lanes q = 0); the three terms in accumulators of their own (chains of two MMAs)
 __device__ __forceinline__ void tile_vec(float (&d)[2][4], const Tile16& X,
                                          const uint2 (&b)[2][2]) {
   float t[3][2][4];
@@ -606,6 +827,66 @@ __device__ __forceinline__ void tile_vec(float (&d)[2][4], const Tile16& X,
     for (int e = 0; e < 4; ++e) d[mt][e] = (t[0][mt][e] + t[1][mt][e]) + t[2][mt][e];
 }
 
+// the rows of d (lanes q = 0) as right-hand side block k
+__device__ __forceinline__ void rhs_terms(__half* hv, int k, const float (&d)[2][4], int lane) {
+  if ((lane & 3) == 0) {
+    __half* v = hv + 128 * k + (lane >> 2);
+#pragma unroll
+    for (int h = 0; h < 4; ++h)  // rows g + 8 h
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const float f = d[h >> 1][2 * (h & 1) + c];
+        const __half hi = __float2half_rn(f);
+        v[64 * c + 8 * h] = hi;
+        v[64 * c + 32 + 8 * h] = __float2half_rn(f - __half2float(hi));
+      }
+  }
+  __syncwarp();
+}
+
+// d := rows of block k minus d
+__device__ __forceinline__ void rhs_minus(const float* rx, const float* ry, int k,
+                                          float (&d)[2][4], int lane) {
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    const int i = 32 * k + (lane >> 2) + 8 * h;
+    d[h >> 1][2 * (h & 1)] = rx[i] - d[h >> 1][2 * (h & 1)];
+    d[h >> 1][2 * (h & 1) + 1] = ry[i] - d[h >> 1][2 * (h & 1) + 1];
+  }
+}
+__device__ __forceinline__ void rhs_store(float* rx, float* ry, int k, const float (&d)[2][4],
+                                          int lane) {
+  if ((lane & 3) == 0) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const int i = 32 * k + (lane >> 2) + 8 * h;
+      rx[i] = d[h >> 1][2 * (h & 1)];
+      ry[i] = d[h >> 1][2 * (h & 1) + 1];
+    }
+  }
+}
+
+// tile_vec of a tile in shared memory, its registers loaded as they are needed
+__device__ __forceinline__ void tile_vec_at(float (&d)[2][4], const uint4* p, int lane,
+                                            const uint2 (&b)[2][2]) {
+  float t[3][2][4];
+#pragma unroll
+  for (int e = 0; e < 24; ++e) t[e >> 3][(e >> 2) & 1][e & 3] = 0.f;
+#pragma unroll
+  for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt) {
+      const uint4 hi = p[32 * (2 * mt + ks) + lane], lo = p[32 * (4 + 2 * mt + ks) + lane];
+      mma_f16(t[0][mt], lo, b[0][ks].x, b[0][ks].y);
+      mma_f16(t[1][mt], hi, b[1][ks].x, b[1][ks].y);
+      mma_f16(t[2][mt], hi, b[0][ks].x, b[0][ks].y);
+    }
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) d[mt][e] = (t[0][mt][e] + t[1][mt][e]) + t[2][mt][e];
+}
+
 __device__ __forceinline__ void cp_async16(void* smem, const void* g) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
                    (unsigned)__cvta_generic_to_shared(smem)),
@@ -613,35 +894,20 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* g) {
                : "memory");
 }
 
-// rows of block n of the right-hand sides: minus d, or d
-__device__ __forceinline__ void rhs_put(float* rx, float* ry, const float (&d)[2][4],
-                                        bool subtract, int lane) {
-  if ((lane & 3) == 0) {
-    float* x = rx + (lane >> 2);
-    float* y = ry + (lane >> 2);
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {  // rows g + 8 h
-      const float vx = d[h >> 1][2 * (h & 1)], vy = d[h >> 1][2 * (h & 1) + 1];
-      x[8 * h] = subtract ? x[8 * h] - vx : vx;
-      y[8 * h] = subtract ? y[8 * h] - vy : vy;
-    }
-  }
-  __syncwarp();
-}
-
-// Block substitution over the tiles: forward (L y = r) or backward (L^T x = y).  Warp 0
-// runs the serial chain: it takes block n - 1's solution off block n and multiplies by
-// the inverse of the diagonal tile; its two tiles per step come through a ring of three
-// stages in shared memory (asynchronous copies, each lane its own elements).  After the
-// barrier that publishes block k's solution the other warps take it off blocks k + 2 and
-// on (each block with its warp), their next tile loaded a step ahead.  One barrier per
-// step.  ring: null when the tiles are in shared memory themselves.
-constexpr int RING_STAGES = 3;
-constexpr size_t RING_BYTES = (size_t)RING_STAGES * 2 * TILE16 * sizeof(uint4);
+// Block substitution over the tiles: forward (L y = r) or backward (L^T x = y).  Warps 0
+// and 1 run the serial chain in turns: step k takes block k - 1's solution off block k and
+// multiplies by the inverse of the diagonal tile, while the other of the two has its tiles
+// for step k + 1 copied to shared memory (buf, 512 elements of 16 bytes each; every lane
+// its own elements) and transposes them there.  Meanwhile the other warps take block
+// k - 1's solution off blocks k + 1 and on (each block with its warp), the next tile loaded
+// behind the products of the one before.  One barrier per step.  Solutions pass between
+// the warps as FP16 terms (hv), converted once by the warp that finds them.  (One chain
+// warp that also fetched its tiles and converted on every read took 2 300 cycles per step,
+// 1 000 of them for this.)  buf: null when the tiles are in shared memory themselves.
 template <int NT, bool BACK>
-__device__ __noinline__ void tri_solve(const uint4* LP, int T, float* rx, float* ry,
-                                       uint4* ring) {
-  constexpr int NO = NT / 32 - 1;  // warps beside the chain's
+__device__ __noinline__ void tri_solve(const uint4* LP, int T, float* rx, float* ry, __half* hv,
+                                       uint4* buf) {
+  constexpr int NO = NT / 32 - 2;  // warps beside the chain's
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   // blocks in the order of the substitution: n-th block
   auto blk = [&](int n) { return BACK ? T - 1 - n : n; };
@@ -650,71 +916,88 @@ __device__ __noinline__ void tri_solve(const uint4* LP, int T, float* rx, float*
   };
   uint2 b[2][2];
   float d[2][4];
-  if (wid == 0) {
-    auto issue = [&](int n) {
-      if (ring != nullptr && n < T) {
-        uint4* dst = ring + (n % RING_STAGES) * 2 * TILE16;
-        const uint4* w = LP + tile_at(blk(n), blk(n));
+  if (wid < 2) {
+    uint4* W = buf + wid * 2 * TILE16;
+    uint4* X = W + TILE16;
+    auto fetch = [&](int n) {  // start copying the tiles of step n
+      if (buf == nullptr || n >= T) return;
+      const uint4* w = LP + tile_at(blk(n), blk(n)) + lane;
+      const uint4* x = LP + tile_of(n, n > 0 ? n - 1 : 0) + lane;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) cp_async16(dst + 32 * e + lane, w + 32 * e + lane);
-        if (n > 0) {
-          const uint4* x = LP + tile_of(n, n - 1);
-#pragma unroll
-          for (int e = 0; e < 8; ++e)
-            cp_async16(dst + TILE16 + 32 * e + lane, x + 32 * e + lane);
+      for (int e = 0; e < 8; ++e) {
+        cp_async16(W + 32 * e + lane, w + 32 * e);
+        cp_async16(X + 32 * e + lane, x + 32 * e);
+      }
+    };
+    auto ready = [&]() {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      if (BACK && buf != nullptr) {
+#pragma unroll 1
+        for (int q = 0; q < 2; ++q) {
+          Tile16 t;
+          t.load(W + q * TILE16, lane);
+          t.transpose();
+          t.store(W + q * TILE16, lane);
         }
       }
-      asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    issue(0);
-    issue(1);
-    for (int n = 0; n < T; ++n) {
-      issue(n + 2);
-      asm volatile("cp.async.wait_group %0;" ::"n"(RING_STAGES - 1) : "memory");
-      const uint4* src = ring + (n % RING_STAGES) * 2 * TILE16;
-      Tile16 X, W;
-      W.load(ring != nullptr ? src : LP + tile_at(blk(n), blk(n)), lane);
-      if (BACK) W.transpose();
-      float* bx = rx + 32 * blk(n);
-      float* by = ry + 32 * blk(n);
-      if (n > 0) {
-        X.load(ring != nullptr ? src + TILE16 : LP + tile_of(n, n - 1), lane);
-        if (BACK) X.transpose();
-        __syncthreads();  // block n - 1 is published, the earlier ones are off block n
-        tile_vec(d, X, b);
-        rhs_put(bx, by, d, true, lane);
+    auto product = [&](const uint4* at, int tile) {
+      if (buf != nullptr) {
+        tile_vec_at(d, at, lane, b);
+      } else {
+        Tile16 t;
+        t.load(LP + tile, lane);
+        if (BACK) t.transpose();
+        tile_vec(d, t, b);
       }
-      rhs_frags(bx, by, lane, b);
-      tile_vec(d, W, b);
-      __syncwarp();
-      rhs_put(bx, by, d, false, lane);
-      rhs_frags(bx, by, lane, b);
+    };
+    fetch(wid);
+    ready();
+    for (int k = 0; k < T; ++k) {
+      if ((k & 1) == wid) {
+        if (k > 0) {
+          rhs_frags(hv, blk(k - 1), lane, b);
+          product(X, tile_of(k, k - 1));
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) d[e >> 2][e & 3] = 0.f;
+        }
+        rhs_minus(rx, ry, blk(k), d, lane);
+        rhs_terms(hv, blk(k), d, lane);
+        rhs_frags(hv, blk(k), lane, b);
+        product(W, tile_at(blk(k), blk(k)));
+        __syncwarp();
+        rhs_terms(hv, blk(k), d, lane);
+        rhs_store(rx, ry, blk(k), d, lane);
+        fetch(k + 2);
+      } else if (k > 0) {
+        ready();
+      }
+      __syncthreads();  // block k is published, block k - 1 is off the blocks after
     }
-    __syncthreads();
   } else {
     // this warp's first block from block n on
-    auto first_of = [&](int n) { return n + (wid - 1 - n % NO + NO) % NO; };
-    Tile16 X, N;
+    auto first_of = [&](int n) { return n + (wid - 2 - n % NO + NO) % NO; };
+    Tile16 N;
     int n0 = first_of(2);
-    if (n0 < T) X.load(LP + tile_of(n0, 0), lane);
-    for (int k = 0; k < T; ++k) {
-      const int n1 = first_of(k + 3);
-      if (n1 < T) N.load(LP + tile_of(n1, k + 1), lane);
-      if (BACK) X.transpose();
-      __syncthreads();  // block k is published
-      if (n0 < T) {
-        rhs_frags(rx + 32 * blk(k), ry + 32 * blk(k), lane, b);
-        tile_vec(d, X, b);
-        rhs_put(rx + 32 * blk(n0), ry + 32 * blk(n0), d, true, lane);
-        for (int n = n0 + NO; n < T; n += NO) {
-          X.load(LP + tile_of(n, k), lane);
-          if (BACK) X.transpose();
-          tile_vec(d, X, b);
-          rhs_put(rx + 32 * blk(n), ry + 32 * blk(n), d, true, lane);
-        }
+    if (n0 < T) N.load(LP + tile_of(n0, 0), lane);
+    __syncthreads();
+    for (int k = 1; k < T; ++k) {
+      const int n1 = first_of(k + 2);
+      if (n0 < T) rhs_frags(hv, blk(k - 1), lane, b);
+      for (int n = n0; n < T; n += NO) {
+        if (BACK) N.transpose();
+        tile_vec(d, N, b);
+        if (n + NO < T)
+          N.load(LP + tile_of(n + NO, k - 1), lane);
+        else if (n1 < T)
+          N.load(LP + tile_of(n1, k), lane);
+        rhs_minus(rx, ry, blk(n), d, lane);
+        __syncwarp();
+        rhs_store(rx, ry, blk(n), d, lane);
       }
-      X = N;
       n0 = n1;
+      __syncthreads();
     }
   }
 }
@@ -724,7 +1007,8 @@ __device__ __noinline__ void tri_solve(const uint4* LP, int T, float* rx, float*
 // [1, 2) for the FP16 terms.
 template <int NT>
 __device__ void chol_solve2(const uint4* LP, int m, const float* dsc, float* rx, float* ry,
-                            double* sh, uint4* ring) {
+                            double* sh, __half* hv,
+                            uint4* buf) {
   const int T = (m + 31) / 32;
   float mx = 0.f, my = 0.f;
   for (int i = threadIdx.x; i < m; i += NT) {
@@ -741,8 +1025,8 @@ __device__ void chol_solve2(const uint4* LP, int m, const float* dsc, float* rx,
     ry[i] = ldexpf(ry[i], -ey);
   }
   __syncthreads();
-  tri_solve<NT, false>(LP, T, rx, ry, ring);
-  tri_solve<NT, true>(LP, T, rx, ry, ring);
+  tri_solve<NT, false>(LP, T, rx, ry, hv, buf);
+  tri_solve<NT, true>(LP, T, rx, ry, hv, buf);
   for (int i = threadIdx.x; i < m; i += NT) {
     rx[i] = ldexpf(rx[i] * dsc[i], ex);
     ry[i] = ldexpf(ry[i] * dsc[i], ey);
@@ -754,7 +1038,7 @@ __device__ void chol_solve2(const uint4* LP, int m, const float* dsc, float* rx,
 struct MpLayout {
   int np;        // n rounded up to 32
   size_t d_off;  // doubles: V 3n, xc n, yc n, Y/C 3n, W 4n
-  size_t f2_off; // float2: zx, zy, gx, gy (np each)
+  size_t f2_off; // float4: z, g (np each)
   size_t f_off;  // float: vx, vy, rx, ry (np each)
   size_t i2_off; // int2: lattice coordinates (np)
   size_t p_off;  // panel: panel_bytes(warps)
@@ -824,10 +1108,8 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   double* yc = xc + n;
   double* YC = yc + n;  // Y = A V (3 n), then C = (Q^T A Q)[0:3, 3:] (3 n)
   double* W = YC + 3 * n;  // 4 n: QR scratch, Z, then t / w
-  float2* zx2 = reinterpret_cast<float2*>(smraw + lay.f2_off);
-  float2* zy2 = zx2 + lay.np;
-  float2* gx2 = zy2 + lay.np;
-  float2* gy2 = gx2 + lay.np;
+  float4* z4 = reinterpret_cast<float4*>(smraw + lay.f2_off);  // (x hi, y hi, x lo, y lo)
+  float4* g4 = z4 + lay.np;
   float* vx = reinterpret_cast<float*>(smraw + lay.f_off);
   float* vy = vx + lay.np;
   float* rx = vy + lay.np;
@@ -835,7 +1117,6 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   int2* cxy = reinterpret_cast<int2*>(smraw + lay.i2_off);
   float* panel = reinterpret_cast<float*>(smraw + lay.p_off);
 
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   float2* B2 = reinterpret_cast<float2*>(matrices + mat_off[sd]);
 
   if (threadIdx.x == 0)
@@ -848,105 +1129,77 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   }
   __syncthreads();
   const bool lat = s_lat != 0;
-  // Centres on the lattice: cxy becomes the grid indices ((2x - 2x_0) / gx,
-  // (2y - 2y_0) / gy) of the grid of steps (gx, gy) through them, and, when every
-  // offset of the grid's extent fits, tab holds the (hi, lo) kernel value of each
-  // offset (a, b) at tab[b tw + a] (tw = 0: no table).  The table lives in W's last n
-  // doubles, free until the refinement.
-  int gx = 1, gy = 1, tw = 0;
-  float2* tab = reinterpret_cast<float2*>(W + 3 * n);
-  const int tsz32 = (int)(table_size < (int64_t)INT_MAX ? table_size : (int64_t)INT_MAX);
+  // Centres on the lattice: with x = 2 p + e in half pixels (e = 0, 1) and g the greatest
+  // common divisor of the whole pixels p - p_0 = g a along an axis, an offset of two centres
+  // is 2 g k + s, s = -1, 0, 1 (the window grid, or half a pixel off it where the window
+  // shift was odd).  When the (hi, lo) kernel values of all these offsets fit the panel, cxy
+  // becomes the codes 3 a + e, whose differences 3 k + s index the table (a when every e is
+  // the same, differences k); otherwise it keeps the lattice coordinates.
+  KEntries K{cxy,
+             reinterpret_cast<const float2*>(panel + NW * 96 * 2),
+             0,
+             phi_table2,
+             (int)(table_size < (int64_t)INT_MAX ? table_size : (int64_t)INT_MAX),
+             xc,
+             yc,
+             phi_table,
+             table_size};
+  int3 dec_x = make_int3(1, 0, 0), dec_y = dec_x;  // lattice coordinate of a code: see lat_of
   if (lat) {
     const int2 o = cxy[0];
-    int v[6];
+    int v[6], w[6];  // whole pixels; w[2..5]: extremes of the half-pixel parts
     lat_grid_init(v);
-    for (int i = threadIdx.x; i < N; i += NT) lat_grid_add(v, cxy[i].x - o.x, cxy[i].y - o.y);
+    lat_grid_init(w);
+    for (int i = threadIdx.x; i < N; i += NT) {
+      lat_grid_add(v, (cxy[i].x >> 1) - (o.x >> 1), (cxy[i].y >> 1) - (o.y >> 1));
+      lat_grid_add(w, cxy[i].x & 1, cxy[i].y & 1);
+    }
     lat_grid_block(v, reinterpret_cast<int*>(sh));
-    const LatTable g = lat_table_of(v, n, tsz32);
-    gx = g.gx;
-    gy = g.gy;
-    for (int i = threadIdx.x; i < N; i += NT)
-      cxy[i] = make_int2((cxy[i].x - o.x) / gx, (cxy[i].y - o.y) / gy);
-    if (g.ok && phi_table2 != nullptr) {
-      tw = g.wx;
-      for (int e = threadIdx.x; e < g.wx * g.wy; e += NT) {
-        const int b = e / g.wx, a = e - b * g.wx;
-        tab[e] = phi_table2[(gy * b) * (gy * b) + (gx * a) * (gx * a)];
+    lat_grid_block(w, reinterpret_cast<int*>(sh));
+    const LatTable g = lat_table_of(v, INT_MAX, INT_MAX);
+    const bool jx = w[2] != w[3], jy = w[4] != w[5];
+    const int64_t wx = jx ? 3 * (int64_t)g.wx - 1 : g.wx, wy = jy ? 3 * (int64_t)g.wy - 1 : g.wy;
+    const int64_t ex = 2 * (int64_t)g.gx * (g.wx - 1) + 1, ey = 2 * (int64_t)g.gy * (g.wy - 1) + 1;
+    if (g.ok && phi_table2 != nullptr && wx * wy <= panel_table(NW) && ex <= 32767 &&
+        ey <= 32767 && ex * ex + ey * ey < (int64_t)K.tsz32) {
+      K.tw = (int)wx;
+      dec_x = make_int3(2 * g.gx, jx, w[2]);
+      dec_y = make_int3(2 * g.gy, jy, w[4]);
+      const int px0 = (o.x >> 1) + v[2], py0 = (o.y >> 1) + v[4];
+      for (int i = threadIdx.x; i < N; i += NT) {
+        const int2 c = cxy[i];
+        const int ax = ((c.x >> 1) - px0) / g.gx, ay = ((c.y >> 1) - py0) / g.gy;
+        cxy[i] = make_int2(jx ? 3 * ax + (c.x & 1) : ax, jy ? 3 * ay + (c.y & 1) : ay);
+      }
+      // offset of a code difference d >= 0: 2 g k + s, d = 3 k + s (or 2 g d)
+      auto offset = [](int d, int3 dec) {
+        if (!dec.y) return dec.x * d;
+        const int k = (d + 1) / 3;
+        return dec.x * k + (d - 3 * k);
+      };
+      float2* tab = const_cast<float2*>(K.tab);
+      for (int e = threadIdx.x; e < (int)(wx * wy); e += NT) {
+        const int b = e / (int)wx, a = e - b * (int)wx;
+        const int dx = offset(a, dec_x), dy = offset(b, dec_y);
+        tab[e] = phi_table2[dy * dy + dx * dx];
       }
     }
     __syncthreads();
   }
-  // A = K + lam I, entry (r, c); on the lattice 4 r^2 is an integer table index
+  const int kmode = !lat || phi_table2 == nullptr ? K_DIRECT : K.tw > 0 ? K_TABLE : K_GATHER;
+  // A = K + lam I, entry (r, c), FP64; on the lattice 4 r^2 is an integer table index
+  auto lat_of = [](int c, int3 dec) { return dec.y ? dec.x * (c / 3) + c % 3 : dec.x * c; };
   auto a_entry = [&](int r, int c) -> double {
     if (r == c) return lam;
     if (lat) {
       const int2 ca = cxy[r], cb = cxy[c];
-      const int64_t dx = (int64_t)gx * (ca.x - cb.x), dy = (int64_t)gy * (ca.y - cb.y);
+      const int64_t dx = lat_of(ca.x, dec_x) - lat_of(cb.x, dec_x);
+      const int64_t dy = lat_of(ca.y, dec_y) - lat_of(cb.y, dec_y);
       const int64_t kq = dy * dy + dx * dx;
       if (kq < table_size) return __ldg(phi_table + kq);
       return phi_pair(xc[r], yc[r], xc[c], yc[c], nullptr, 0);
     }
     return phi_pair(xc[r], yc[r], xc[c], yc[c], phi_table, table_size);
-  };
-  // the same entry as a (hi, lo) float pair; ci = lattice coordinates of centre i
-  const float2 lam2 = df_split(lam);
-  auto a_entry_df = [&](int i, int2 ci, int j) -> float2 {
-    if (i == j) return lam2;
-    if (lat) {
-      const int2 cj = cxy[j];
-      const int64_t dx = (int64_t)gx * (ci.x - cj.x), dy = (int64_t)gy * (ci.y - cj.y);
-      const int64_t kq = dy * dy + dx * dx;
-      if (kq < table_size)
-        return phi_table2 != nullptr ? phi_table2[kq] : df_split(__ldg(phi_table + kq));
-      return df_split(phi_pair(xc[i], yc[i], xc[j], yc[j], nullptr, 0));
-    }
-    return df_split(phi_pair(xc[i], yc[i], xc[j], yc[j], phi_table, table_size));
-  };
-  // entries (i, j0 .. j0 + cnt - 1) of A as pairs (0 < cnt <= 8, the rest zero): on the
-  // lattice the eight table loads are issued before any is used (the loads, mostly
-  // L2 hits, bound these phases), the diagonal and far entries patched afterwards
-  auto a_batch_df = [&](int i, int2 ci, int j0, int cnt, float2(&out)[8]) {
-    if (lat && tw > 0) {  // every offset in the shared table
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int2 cj = cxy[j0 + min(u, cnt - 1)];
-        out[u] = tab[abs(ci.y - cj.y) * tw + abs(ci.x - cj.x)];
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (u >= cnt)
-          out[u] = make_float2(0.f, 0.f);
-        else if (j0 + u == i)
-          out[u] = lam2;
-      }
-    } else if (lat && phi_table2 != nullptr) {
-      // 4 r^2 in 32-bit integers: the lattice coordinates are below 2^30 in magnitude,
-      // so their differences fit, and |dx|, |dy| <= 32767 keeps dx^2 + dy^2 below
-      // 2^31; farther pairs (beyond the table anyway) take the direct kernel value
-      int kq[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int2 cj = cxy[j0 + min(u, cnt - 1)];
-        const int dx = gx * (ci.x - cj.x), dy = gy * (ci.y - cj.y);
-        const bool near = (unsigned)dx + 32767u <= 65534u && (unsigned)dy + 32767u <= 65534u;
-        kq[u] = near ? dy * dy + dx * dx : INT_MAX;
-        out[u] = phi_table2[kq[u] < tsz32 ? kq[u] : 0];
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int j = j0 + u;
-        if (u >= cnt)
-          out[u] = make_float2(0.f, 0.f);
-        else if (j == i)
-          out[u] = lam2;
-        else if (kq[u] >= tsz32)
-          out[u] = df_split(phi_pair(xc[i], yc[i], xc[j], yc[j], nullptr, 0));
-      }
-    } else {
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        out[u] = (u < cnt) ? a_entry_df(i, ci, j0 + u) : make_float2(0.f, 0.f);
-    }
   };
 
   // ---- Householder QR of P = [1, y, x] (FP64), V rows k hold v_k (zeros above k).  The
@@ -1029,101 +1282,26 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   double* Y0 = YC;
   double* Y1 = YC + n;
   double* Y2 = YC + 2 * n;
-  // V and Z as (hi, lo) float pairs, [3][np] each: the f2 and f regions (6 np pairs)
-  // are free until the refinement
-  float2* Vd = zx2;
-  float2* Zd = zx2 + 3 * lay.np;
+  // the pairs of V for Y, then the columns of the projection: the f2 and f regions (48 np
+  // bytes) are free until the refinement
+  float4* pairs = reinterpret_cast<float4*>(smraw + lay.f2_off);
   const int np = lay.np;
-  for (int i = threadIdx.x; i < np; i += NT) {
-    const bool in = i < N;
-    Vd[i] = in ? df_split(V0[i]) : make_float2(0.f, 0.f);
-    Vd[np + i] = in ? df_split(V1[i]) : make_float2(0.f, 0.f);
-    Vd[2 * np + i] = in ? df_split(V2[i]) : make_float2(0.f, 0.f);
+  for (int i = threadIdx.x; i < N; i += NT) {
+    const float2 a = df_split(V1[i]), b = df_split(V2[i]);
+    pairs[i] = make_float4(a.x, b.x, a.y, b.y);
   }
   __syncthreads();
   // every CTA of the cluster has started (and holds its V) before any CTA writes
   // into a peer's shared memory below
   cluster.sync();
-  // ---- Y = A V in double-float on the FP32 pipe.  A is symmetric: lane = column c,
-  // the rows r in chunks (jobs = column block x chunk, a multiple of the warp count
-  // when the scratch allows); the chunks' partial sums are added in a fixed order.
-  // The column blocks are spread over the cluster's CTAs; each Y value is rounded to
-  // double and written into every CTA's Y.
   {
-    auto write_y = [&](int c, float2 s0, float2 s1, float2 s2) {
-      const double y0 = df_to_double(s0), y1 = df_to_double(s1), y2 = df_to_double(s2);
-      for (int q = 0; q < csize; ++q) {
-        double* Yq = (q == crank) ? YC : cluster.map_shared_rank(YC, q);
-        Yq[c] = y0;
-        Yq[n + c] = y1;
-        Yq[2 * n + c] = y2;
-      }
-    };
-    const int ncb = (N + 31) / 32;
-    const int nloc = (crank < ncb) ? (ncb - crank + csize - 1) / csize : 0;
-    int rs = 1;
-    if (nloc > 0) {
-      int a = nloc, b = NW;
-      while (b != 0) {
-        const int t = a % b;
-        a = b;
-        b = t;
-      }
-      rs = NW / a;  // nloc * rs is a multiple of NW
-      const int max_jobs = (int)(panel_bytes(NW) / (96 * sizeof(float2)));
-      while (rs > 1 && (nloc * rs > max_jobs || 8 * rs > N)) rs >>= 1;
-    }
-    float2* part = reinterpret_cast<float2*>(panel);  // [job][3][32]
-    for (int j = wid; j < nloc * rs; j += NW) {
-      const int l = j / rs, ch = j - l * rs;
-      const int c = 32 * (crank + csize * l) + lane;
-      const int r0 = (int)((int64_t)N * ch / rs), r1 = (int)((int64_t)N * (ch + 1) / rs);
-      // sums of V0 and V1 in the lanes of (h01, l01) (packed FP32x2), V2 in (h2, l2)
-      float2 h01 = make_float2(0.f, 0.f), l01 = make_float2(0.f, 0.f);
-      float h2 = 0.f, l2 = 0.f;
-      if (c < N) {
-        const int2 cc = cxy[c];
-        for (int rb = r0; rb < r1; rb += 8) {
-          const int cnt = min(8, r1 - rb);
-          float2 a[8];
-          a_batch_df(c, cc, rb, cnt, a);
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            if (u < cnt) {
-              const int r = rb + u;
-              const float2 v0 = Vd[r], v1 = Vd[np + r];
-              df_mac_x2(a[u], make_float2(v0.x, v1.x), make_float2(v0.y, v1.y), h01, l01);
-              df_mac(a[u], Vd[2 * np + r], h2, l2);
-            }
-          }
-        }
-      }
-      const float h0 = h01.x, l0 = l01.x, h1 = h01.y, l1 = l01.y;
-      if (rs == 1) {
-        if (c < N) write_y(c, make_float2(h0, l0), make_float2(h1, l1), make_float2(h2, l2));
-      } else {
-        part[(3 * j + 0) * 32 + lane] = make_float2(h0, l0);
-        part[(3 * j + 1) * 32 + lane] = make_float2(h1, l1);
-        part[(3 * j + 2) * 32 + lane] = make_float2(h2, l2);
-      }
-    }
-    if (rs > 1) {
-      __syncthreads();
-      for (int t = threadIdx.x; t < nloc * 32; t += NT) {
-        const int l = t >> 5, ln = t & 31;
-        const int c = 32 * (crank + csize * l) + ln;
-        if (c >= N) continue;
-        const float2* pj = part + (size_t)3 * 32 * (l * rs);
-        float2 s0 = pj[ln], s1 = pj[32 + ln], s2 = pj[64 + ln];
-        for (int ch = 1; ch < rs; ++ch) {
-          pj += 3 * 32;
-          s0 = df_add(s0, pj[ln]);
-          s1 = df_add(s1, pj[32 + ln]);
-          s2 = df_add(s2, pj[64 + ln]);
-        }
-        write_y(c, s0, s1, s2);
-      }
-    }
+    float2* part = reinterpret_cast<float2*>(panel);
+    if (kmode == K_TABLE)
+      build_y<NT, K_TABLE>(K, pairs, V, V0[0], lam, N, n, YC, part);
+    else if (kmode == K_GATHER)
+      build_y<NT, K_GATHER>(K, pairs, V, V0[0], lam, N, n, YC, part);
+    else
+      build_y<NT, K_DIRECT>(K, pairs, V, V0[0], lam, N, n, YC, part);
   }
   cluster.sync();
   // ---- Q^T A Q = A - Z V^T - V Z^T (compact WY, Q = H0 H1 H2 = I - V T V^T),
@@ -1186,12 +1364,19 @@ __global__ void __launch_bounds__(NT, 512 / NT)
       Z1[i] = z[1];
       Z2[i] = z[2];
     }
-    for (int i = N + threadIdx.x; i < np; i += NT) Zd[i] = Zd[np + i] = Zd[2 * np + i] = make_float2(0.f, 0.f);
     __syncthreads();
-    for (int i = threadIdx.x; i < N; i += NT) {
-      Zd[i] = df_split(Z0[i]);
-      Zd[np + i] = df_split(Z1[i]);
-      Zd[2 * np + i] = df_split(Z2[i]);
+    float* pf = reinterpret_cast<float*>(pairs);
+    for (int c = threadIdx.x; c < np; c += NT) {  // unknown c: row c + 3 (zero past m)
+      const bool in = c < m;
+      const double src[5] = {in ? -Z0[c + 3] : 0.0, in ? V1[c + 3] : 0.0, in ? V2[c + 3] : 0.0,
+                             in ? Z1[c + 3] : 0.0, in ? Z2[c + 3] : 0.0};
+#pragma unroll
+      for (int k = 0; k < 5; ++k) {
+        const float2 d = df_split(src[k]);
+        float* q = pf + 4 * (k * (np / 2) + (c >> 1)) + (c & 1);
+        q[0] = d.x;
+        q[2] = d.y;
+      }
     }
     __syncthreads();
   }
@@ -1210,79 +1395,16 @@ __global__ void __launch_bounds__(NT, 512 / NT)
       C[k * n + c] = proj(k, c + 3);
     }
   }
-  // B22 by 32 x 32 tiles (I >= J), half a tile (16 columns) at a time: the lower
-  // entries are written by columns, then mirrored through a per-warp shared tile.
+  // ---- B22 in double-float
+  const BPairs B{B2, m, mp, m > 32 * SMALL_T};
   {
-    float2* S = reinterpret_cast<float2*>(panel) + wid * 16 * 33;
-    const int T = (m + 31) / 32;
-    const int npairs = T * (T + 1) / 2;
-    for (int pidx = crank * NW + wid; pidx < npairs; pidx += csize * NW) {
-      int I = (int)((sqrtf(8.f * pidx + 1.f) - 1.f) * 0.5f);
-      while ((I + 1) * (I + 2) / 2 <= pidx) ++I;
-      while (I * (I + 1) / 2 > pidx) --I;
-      const int J = pidx - I * (I + 1) / 2;
-      const int r = 32 * I + lane;
-      // the row's -Z_k and -V_k pairs and lattice coordinates
-      const int rg = (r < m) ? r + 3 : 3;
-      const int2 cr = cxy[rg];
-      float2 nz[3], nv[3];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const float2 zv = Zd[k * np + rg], vv = Vd[k * np + rg];
-        nz[k] = make_float2(-zv.x, -zv.y);
-        nv[k] = make_float2(-vv.x, -vv.y);
-      }
-      for (int h = 0; h < 2; ++h) {
-        for (int qb = 0; qb < 16; qb += 8) {
-          const int c0 = 32 * J + 16 * h + qb;
-          if (c0 >= m) break;
-          const int cnt = min(8, m - c0);
-          float2 a[8];
-          a_batch_df(rg, cr, c0 + 3, cnt, a);
-          // A - Z V^T - V Z^T in double-float: entries of A up to ~1e5 cancel to B
-          // entries ~1e2-1e4; the ~2^-48 |A| rounding leaves B within ~1e-11 of its
-          // FP64 value, the interpolated field within ~1e-9 px.  Columns c, c + 1 in
-          // the lanes of float2 pairs (packed FP32x2 instructions).
-#pragma unroll
-          for (int u = 0; u < 8; u += 2) {
-            const int c = c0 + u;
-            const bool in0 = u < cnt && r < m && r >= c;
-            const bool in1 = u + 1 < cnt && r < m && r >= c + 1;
-            if (in0 || in1) {
-              const int cg0 = c + 3, cg1 = min(c + 4, N - 1);
-              float2 sh = make_float2(a[u].x, a[u + 1].x), sl = make_float2(a[u].y, a[u + 1].y);
-#pragma unroll
-              for (int k = 0; k < 3; ++k) {
-                const float2 v0 = Vd[k * np + cg0], v1 = Vd[k * np + cg1];
-                const float2 z0 = Zd[k * np + cg0], z1 = Zd[k * np + cg1];
-                df_mac_x2(nz[k], make_float2(v0.x, v1.x), make_float2(v0.y, v1.y), sh, sl);
-                df_mac_x2(nv[k], make_float2(z0.x, z1.x), make_float2(z0.y, z1.y), sh, sl);
-              }
-              const float2 hi = __fadd2_rn(sh, sl);
-              const float2 lo = __fadd2_rn(sl, df_neg2(__fadd2_rn(hi, df_neg2(sh))));
-              if (in0) {
-                const float2 sv = make_float2(hi.x, lo.x);
-                __stcs(B2 + (int64_t)c * mp + r, sv);  // streaming: keeps L2 for the factor
-                S[(qb + u) * 33 + lane] = sv;
-              }
-              if (in1) {
-                const float2 sv = make_float2(hi.y, lo.y);
-                __stcs(B2 + (int64_t)(c + 1) * mp + r, sv);
-                S[(qb + u + 1) * 33 + lane] = sv;
-              }
-            }
-          }
-        }
-        __syncwarp();
-#pragma unroll 4
-        for (int st = 0; st < 16; ++st) {
-          const int rr = 2 * st + (lane >> 4), qq = lane & 15;
-          const int r2 = 32 * I + rr, c2 = 32 * J + 16 * h + qq;
-          if (r2 < m && c2 < m && r2 > c2) __stcs(B2 + (int64_t)r2 * mp + c2, S[qq * 33 + rr]);
-        }
-        __syncwarp();
-      }
-    }
+    const float2 lam2 = df_split(lam);
+    if (kmode == K_TABLE)
+      build_b<NT, K_TABLE>(K, pairs, np, lam2, B, crank, csize);
+    else if (kmode == K_GATHER)
+      build_b<NT, K_GATHER>(K, pairs, np, lam2, B, crank, csize);
+    else
+      build_b<NT, K_DIRECT>(K, pairs, np, lam2, B, crank, csize);
   }
   cluster.sync();  // the cluster's B tiles are in global memory, visible to rank 0
   if (crank != 0) return;
@@ -1291,7 +1413,7 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   if (threadIdx.x == 0) s_flag = 0;
   __syncthreads();
   for (int i = threadIdx.x; i < m; i += NT) {
-    const float v = B2[(int64_t)i * mp + i].x;
+    const float v = B.at(i, i).x;
     if (!(v > 0.f)) s_flag = 1;
     dsc[i] = (v > 0.f) ? ldexpf(1.f, -(ilogbf(v) >> 1)) : 1.f;
   }
@@ -1299,8 +1421,18 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   uint4* LP = (m <= 32 * SMALL_T)
                   ? reinterpret_cast<uint4*>(smraw + lay.p_off + ((CHOL_SMEM + 15) & ~(size_t)15))
                   : reinterpret_cast<uint4*>(matrices32 + mat_off[sd]);
-  if (!chol_factor<NT>(B2, m, mp, dsc, LP, panel, &s_flag)) return;
-  uint4* ring = (m <= 32 * SMALL_T) ? nullptr : reinterpret_cast<uint4*>(panel);
+  if (!chol_factor<NT>(B, dsc, LP, panel, &s_flag)) return;
+  // the residual: staging of the warps, then the tile products, in the panel when they fit,
+  // else behind the tiles of B in its slot (from 7 tile rows on (m + 6)^2 pairs hold both)
+  float2* stage = reinterpret_cast<float2*>(panel);
+  constexpr size_t STAGE_BYTES = (size_t)NW * 16 * 33 * sizeof(float2);
+  const int nT = (m + 31) / 32;
+  float4* part = (STAGE_BYTES + residual_part_bytes(nT, NW / 8) <= panel_bytes(NW))
+                     ? reinterpret_cast<float4*>(smraw + lay.p_off + STAGE_BYTES)
+                     : reinterpret_cast<float4*>(B2 + (size_t)1024 * (nT * (nT + 1) / 2));
+  // the substitutions' right-hand sides, behind the tiles of small subdomains
+  __half* hv = reinterpret_cast<__half*>(smraw + lay.p_off + HV_OFF);
+  uint4* buf = (m <= 32 * SMALL_T) ? nullptr : reinterpret_cast<uint4*>(panel);
 
   // ---- outlier iterations with refined solves (x and y in lockstep)
   double* wx = W + 2 * n;
@@ -1308,7 +1440,7 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   for (int r = threadIdx.x; r < lay.np; r += NT) {
     vx[r] = (r < N) ? ux[idx[r]] : 0.f;
     vy[r] = (r < N) ? uy[idx[r]] : 0.f;
-    zx2[r] = zy2[r] = make_float2(0.f, 0.f);
+    z4[r] = g4[r] = make_float4(0.f, 0.f, 0.f, 0.f);
     rx[r] = ry[r] = 0.f;
   }
   __syncthreads();
@@ -1351,8 +1483,8 @@ __global__ void __launch_bounds__(NT, 512 / NT)
           s_q1[i] = gxv;
           s_q1[3 + i] = gyv;
         } else {
-          gx2[i - 3] = df_split(gxv);
-          gy2[i - 3] = df_split(gyv);
+          const float2 a = df_split(gxv), b = df_split(gyv);
+          g4[i - 3] = make_float4(a.x, b.x, a.y, b.y);
         }
       }
       __syncthreads();
@@ -1363,26 +1495,33 @@ __global__ void __launch_bounds__(NT, 512 / NT)
     for (int it = 0; it < max_refine; ++it) {
       if (z_zero) {  // z = 0: rho = g
         for (int i = threadIdx.x; i < m; i += NT) {
-          rx[i] = __fadd_rn(gx2[i].x, gx2[i].y);
-          ry[i] = __fadd_rn(gy2[i].x, gy2[i].y);
+          rx[i] = __fadd_rn(g4[i].x, g4[i].z);
+          ry[i] = __fadd_rn(g4[i].y, g4[i].w);
         }
         __syncthreads();
         z_zero = false;
       } else {
-        residual_df2<NT>(B2, m, mp, zx2, zy2, gx2, gy2, rx, ry);
+        if (B.tiles)
+          residual_tiles<NT>(B, z4, g4, rx, ry, part, stage);
+        else
+          residual_small<NT>(B, z4, g4, rx, ry);
       }
-      chol_solve2<NT>(LP, m, dsc, rx, ry, sh, ring);
+      chol_solve2<NT>(LP, m, dsc, rx, ry, sh, hv, buf);
       ++nsweeps;
       float dm = 0.f, zm = 0.f;
       for (int i = threadIdx.x; i < m; i += NT) {
-        if (!done[0]) zx2[i] = df_add(zx2[i], make_float2(rx[i], 0.f));
-        if (!done[1]) zy2[i] = df_add(zy2[i], make_float2(ry[i], 0.f));
+        const float4 zv = z4[i];
+        float2 zh = make_float2(zv.x, zv.y), zl = make_float2(zv.z, zv.w);
+        df_acc_x2(make_float2(done[0] ? 0.f : rx[i], done[1] ? 0.f : ry[i]),
+                  make_float2(0.f, 0.f), zh, zl);
+        df_norm_x2(zh, zl);
+        z4[i] = make_float4(zh.x, zh.y, zl.x, zl.y);
         // (beyond the FP16 range of the factor's products the corrections are not finite:
         // their bits compare as the largest)
         const unsigned ax = done[0] ? 0u : __float_as_uint(fabsf(rx[i]));
         const unsigned ay = done[1] ? 0u : __float_as_uint(fabsf(ry[i]));
         dm = __uint_as_float(max(__float_as_uint(dm), max(ax, ay)));
-        zm = fmaxf(zm, fmaxf(fabsf(zx2[i].x), fabsf(zy2[i].x)));
+        zm = fmaxf(zm, fmaxf(fabsf(zh.x), fabsf(zh.y)));
       }
       const float2 dz = block_max2<NT>(dm, zm, sh);
       if (!(dz.x < INFINITY)) break;  // the FP64 LU takes over
@@ -1417,7 +1556,8 @@ __global__ void __launch_bounds__(NT, 512 / NT)
       double pr[12];
       for (int k = 0; k < 12; ++k) pr[k] = 0.0;
       for (int i = threadIdx.x; i < m; i += NT) {
-        const double zxv = df_to_double(zx2[i]), zyv = df_to_double(zy2[i]);
+        const float4 zv = z4[i];
+        const double zxv = (double)zv.x + (double)zv.z, zyv = (double)zv.y + (double)zv.w;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
           const double cv = C[k * n + i], v = V[k * n + i + 3];
@@ -1443,8 +1583,8 @@ __global__ void __launch_bounds__(NT, 512 / NT)
       }
       __syncthreads();
       for (int i = threadIdx.x; i < N; i += NT) {
-        double a = (i < 3) ? 0.0 : df_to_double(zx2[i - 3]);
-        double b = (i < 3) ? 0.0 : df_to_double(zy2[i - 3]);
+        const float4 zv = i < 3 ? make_float4(0.f, 0.f, 0.f, 0.f) : z4[i - 3];
+        double a = (double)zv.x + (double)zv.z, b = (double)zv.y + (double)zv.w;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
           const double v = V[k * n + i];
