@@ -76,29 +76,49 @@ __device__ __forceinline__ void lat_grid_block(int (&v)[6], int* scratch) {
   __syncthreads();
 }
 
-// Table geometry of a reduced grid: step (gx, gy) >= 1 and the numbers of offsets
-// wx, wy along each axis (offsets 0 .. w - 1 in steps).  Usable when the table fits
-// `capacity` entries and every offset's 4 r^2 = (gx a)^2 + (gy b)^2 stays a 32-bit
-// index below `tsize` (then no pair of the grid falls beyond the lattice table).
-struct LatTable {
-  int gx, gy, wx, wy;
-  bool ok;
+// Codes of lattice coordinates along one axis.  With a coordinate 2 p + e in half pixels
+// (e = 0, 1) and whole pixels p = p_min + g a, the offset of two points is 2 g k + s with
+// s = -1, 0, 1: points on the grid of step g, or half a pixel off it (the midpoints of odd
+// window shifts).  The codes 3 a + e differ by 3 k + s, so a table of one entry per code
+// difference holds every offset; when every e is the same (half = false) the codes are a.
+struct LatCodes {
+  int g, width;  // step in pixels, number of code differences 0 .. width - 1
+  bool half;
+  __device__ __forceinline__ int code(int c, int p_min) const {
+    const int a = ((c >> 1) - p_min) / g;
+    return half ? 3 * a + (c & 1) : a;
+  }
+  // the offset (half pixels, >= 0) of a code difference d >= 0
+  __device__ __forceinline__ int offset(int d) const {
+    if (!half) return 2 * g * d;
+    const int k = (d + 1) / 3;
+    return 2 * g * k + (d - 3 * k);
+  }
+  // a coordinate (half pixels, from the smallest) of a code
+  __device__ __forceinline__ int coord(int c) const {
+    return half ? 2 * g * (c / 3) + c % 3 : 2 * g * c;
+  }
 };
 
-__device__ __forceinline__ LatTable lat_table_of(const int (&v)[6], int64_t capacity,
-                                                 int tsize) {
-  LatTable t;
-  t.gx = v[0] > 0 ? v[0] : 1;
-  t.gy = v[1] > 0 ? v[1] : 1;
-  t.ok = v[2] <= v[3] && v[4] <= v[5];
-  t.wx = t.ok ? (int)(((int64_t)v[3] - v[2]) / t.gx) + 1 : 0;
-  t.wy = t.ok ? (int)(((int64_t)v[5] - v[4]) / t.gy) + 1 : 0;
-  if (t.ok) {
-    const int64_t ex = (int64_t)t.gx * (t.wx - 1), ey = (int64_t)t.gy * (t.wy - 1);
-    t.ok = (int64_t)t.wx * t.wy <= capacity && ex <= 32767 && ey <= 32767 &&
-           ex * ex + ey * ey < (int64_t)tsize;
-  }
-  return t;
+// From the reduced whole pixels (their gcd and extremes, lat_grid_*).
+__device__ __forceinline__ LatCodes lat_codes(int gcd, int pmin, int pmax, bool half) {
+  LatCodes c;
+  c.g = gcd > 0 ? gcd : 1;
+  c.half = half;
+  // (extents beyond 2^15 pixels fail lat_codes_fit: the width saturates)
+  const int64_t a = pmin <= pmax ? ((int64_t)pmax - pmin) / c.g : INT_MAX;
+  const int64_t w = half ? 3 * a + 2 : a + 1;
+  c.width = (int)(w < (1 << 20) ? w : (1 << 20));
+  return c;
+}
+
+// Whether every offset's 4 r^2 is a 32-bit index below `tsize` (then no pair of the grid
+// falls beyond the lattice table).
+__device__ __forceinline__ bool lat_codes_fit(const LatCodes& x, const LatCodes& y, int tsize) {
+  if (x.width >= (1 << 20) || y.width >= (1 << 20)) return false;
+  const int64_t ex = 2 * (int64_t)x.g * ((x.width + 1) / (x.half ? 3 : 1)) + 1;
+  const int64_t ey = 2 * (int64_t)y.g * ((y.width + 1) / (y.half ? 3 : 1)) + 1;
+  return ex <= 32767 && ey <= 32767 && ex * ex + ey * ey < (int64_t)tsize;
 }
 
 }  // namespace fi

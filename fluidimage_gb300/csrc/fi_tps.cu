@@ -697,6 +697,7 @@ __device__ __forceinline__ double coef_norm_hoisted(const double* c, double x, d
 // the subdomain's y band are scanned.  subdoms_from_plan: the grid is a capacity,
 // blocks past the plan's subdomains return; centres_from_plan: the points are the
 // plan's centres (npts a capacity).
+constexpr int MEMBER_AXIS = 1024;  // half pixels of a subdomain along an axis
 __global__ void __launch_bounds__(512)
     k_tps_members(const fi_tps_plan* plan_ptr, const double* px, const double* py, int npts,
                   int mode, int32_t* counts, const int64_t* offsets, int32_t* indices,
@@ -797,6 +798,19 @@ __global__ void __launch_bounds__(512)
     if (lane < nw) warp_tot[lane] = incl - v;
   }
   __syncthreads();
+  // the two factors of coef_norm for every half pixel of the subdomain (the divisions of
+  // every member were bound by the FP64 pipe)
+  __shared__ double fac[2][MEMBER_AXIS];
+  const bool tab = lat && (int64_t)X1 - X0 <= MEMBER_AXIS && (int64_t)Y1 - Y0 <= MEMBER_AXIS;
+  if (tab) {  // 1 - (x - xc)^2 / dxm^2 and the same for y
+    const int wx = max(0, X1 - X0), wy = max(0, Y1 - Y0);
+    for (int t = threadIdx.x; t < wx + wy; t += blockDim.x) {
+      const int ax = t < wx ? 0 : 1, e = t - ax * wx;
+      const double d = __dsub_rn(0.5 * (double)((ax ? Y0 : X0) + e), s_cn[ax]);
+      fac[ax][e] = __dsub_rn(1.0, __ddiv_rn(__dmul_rn(d, d), s_cn[2 + ax]));
+    }
+    __syncthreads();
+  }
   int64_t pos = offsets[i] + warp_tot[wid];
   constexpr int R = 4;  // membership of four chunks of 32 tested (loads issued) first
   for (int c0 = s0; c0 < s1; c0 += R * 32) {
@@ -813,7 +827,12 @@ __global__ void __launch_bounds__(512)
       if (in[r]) {
         const int64_t at = pos + __popc(b & ((1u << lane) - 1u));
         indices[at] = q;
-        coefs[at] = coef_norm_hoisted(s_cn, px[q], py[q]);
+        if (tab) {
+          const int2 XY = reinterpret_cast<const int2*>(xy2)[q];
+          coefs[at] = __dadd_rn(__dmul_rn(fac[0][XY.x - X0], fac[1][XY.y - Y0]), 0.001);
+        } else {
+          coefs[at] = coef_norm_hoisted(s_cn, px[q], py[q]);
+        }
       }
       pos += __popc(b);
     }
@@ -1138,19 +1157,23 @@ __global__ void k_tps_blend_centers(const fi_tps_plan* plan_ptr, const double* c
   outy[q] = __ddiv_rn(sy, nrm);
 }
 
-// Interpolation at the new positions of subdomain blockIdx.y:
+// Interpolation at the new positions of subdomain blockIdx.y
+// (interpolate, thin_plate_spline_subdom.py:224-234):
 // part[k] = coef_k * (sum_j w_j phi(|q_k - c_j|^2) + w_N + w_N+1 y + w_N+2 x).
-// Part of each subdomain's TPS at its new positions: coef * (sum_j w_j phi_j + affine)
-// (interpolate, thin_plate_spline_subdom.py:224-234).  On the lattice with the
-// (hi, lo) table the kernel sum runs in double-float on the FP32 pipe (~1e-14
-// relative per term), else in FP64.  When the block's positions and the centres lie
-// on one grid of the lattice, or the centres half a pixel off it along an axis (the
-// final evaluation, on the grid of the pass's own windows), and the grid's offsets fit
-// tab_cap entries (0 when the launch has no room for them), the block reads the
-// (hi, lo) values of the grid's offsets from shared memory (the same table entries).
-constexpr int EVAL_TABLE = 2048;
+// On the lattice with the (hi, lo) table the kernel sum runs in double-float on the FP32
+// pipe (~1e-14 relative per term; both components in the lanes of packed instructions),
+// else in FP64.  The kernel values come from a table of the block's own in shared memory
+// when the offsets between its positions and the centres are few (lat_codes: a grid of
+// the lattice, or half a pixel off it along an axis), else from the lattice table in
+// memory, whose gathers (a sector per lane) bound that path.  The table is a rectangle
+// (wx x wy offsets) or, where that does not fit and both axes have one step, the triangle
+// of its larger offset (the field of a pass at the next one's positions, on a grid twice
+// as fine as the centres').  65 025 positions of 306 subdomains on the pass's own grid:
+// 185 -> 103 us; the two fields between the passes of a 2048^2 run 290 -> 130 us.
+constexpr int EVAL_TABLE = 9216;
+constexpr int EVAL_NT = 512;
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(EVAL_NT)
     k_tps_eval(const int32_t* counts, const int64_t* offsets, const int32_t* indices,
                const int64_t* w_off, const double* weights, const double* cx, const double* cy,
                const int32_t* ncounts, const int64_t* noffsets, const int32_t* nindices,
@@ -1158,20 +1181,19 @@ __global__ void __launch_bounds__(256)
                double* party, const double* table, const float2* table2, int64_t tsize,
                const int32_t* cxy2, const int32_t* c_on_lattice, int max_members,
                int tab_cap) {
-  extern __shared__ double sh[];
+  extern __shared__ __align__(16) double sh[];
   const int sd = blockIdx.y;
   const int N = counts[sd], n = N + 3, M = ncounts[sd];
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (blockIdx.x * blockDim.x >= M) return;
-  const int NM = max_members;
-  double* scx = sh;
-  double* scy = sh + NM;
-  double* swx = sh + 2 * NM;
-  double* swy = swx + NM + 3;
-  int2* sxy2 = reinterpret_cast<int2*>(swy + NM + 3);   // lattice coordinates of the centres
-  float2* dwx = reinterpret_cast<float2*>(sxy2 + NM);  // weights as (hi, lo) pairs
-  float2* dwy = dwx + NM;
-  float2* tab = dwy + NM;  // tab_cap pairs: kernel values of the grid offsets
+  const int NM = (max_members + 4) & ~1;  // (affine weights behind the centres'; even)
+  float4* dw = reinterpret_cast<float4*>(sh);  // weights: (x hi, y hi, x lo, y lo)
+  double* scx = sh + 2 * NM;
+  double* scy = scx + NM;
+  double* swx = scy + NM;
+  double* swy = swx + NM;
+  int2* code = reinterpret_cast<int2*>(swy + NM);  // lattice coordinates, or codes
+  float2* tab = reinterpret_cast<float2*>(code + NM);  // tab_cap pairs
   __shared__ int s_lat, s_red[6 * 32];
   const int64_t off = offsets[sd];
   const double* w = weights + w_off[sd];
@@ -1180,14 +1202,14 @@ __global__ void __launch_bounds__(256)
     const int a = indices[off + j];
     scx[j] = cx[a];
     scy[j] = cy[a];
-    if (cxy2 != nullptr) sxy2[j] = make_int2(cxy2[2 * a], cxy2[2 * a + 1]);
+    if (cxy2 != nullptr) code[j] = make_int2(cxy2[2 * a], cxy2[2 * a + 1]);
   }
   for (int j = threadIdx.x; j < n; j += blockDim.x) {
     swx[j] = w[j];
     swy[j] = w[n + j];
     if (table2 != nullptr && j < N) {
-      dwx[j] = df_split(w[j]);
-      dwy[j] = df_split(w[n + j]);
+      const float2 a = df_split(w[j]), b = df_split(w[n + j]);
+      dw[j] = make_float4(a.x, b.x, a.y, b.y);
     }
   }
   __syncthreads();
@@ -1199,147 +1221,90 @@ __global__ void __launch_bounds__(256)
   const bool qlat = k < M && s_lat && table != nullptr && X2 == rint(X2) && Y2 == rint(Y2) &&
                     fabs(X2) < 1073741824.0 && fabs(Y2) < 1073741824.0;
   const int tsz32 = (int)(tsize < (int64_t)INT_MAX ? tsize : (int64_t)INT_MAX);
-  // the grid through the centres and the block's lattice positions (origin: the first
-  // centre; every lattice coordinate is below 2^30 in magnitude, so offsets fit)
-  int tw = 0, jw = 0, QA = 0, QB = 0;
+  int2 Q = make_int2(qlat ? (int)X2 : 0, qlat ? (int)Y2 : 0);
+  int tw = 0;  // row length of the table, -1: the triangle, 0: none
   if (s_lat && table != nullptr && table2 != nullptr) {
-    const int2 o = sxy2[0];
-    int v[6];
+    // whole pixels and half-pixel parts of the centres and the block's positions
+    const int2 o = code[0];
+    int v[6], h[6];
     lat_grid_init(v);
-    for (int j = threadIdx.x; j < N; j += blockDim.x) lat_grid_add(v, sxy2[j].x - o.x, sxy2[j].y - o.y);
-    if (qlat) lat_grid_add(v, (int)X2 - o.x, (int)Y2 - o.y);
+    lat_grid_init(h);
+    for (int j = threadIdx.x; j < N; j += blockDim.x) {
+      lat_grid_add(v, (code[j].x >> 1) - (o.x >> 1), (code[j].y >> 1) - (o.y >> 1));
+      lat_grid_add(h, code[j].x & 1, code[j].y & 1);
+    }
+    if (qlat) {
+      lat_grid_add(v, (Q.x >> 1) - (o.x >> 1), (Q.y >> 1) - (o.y >> 1));
+      lat_grid_add(h, Q.x & 1, Q.y & 1);
+    }
     lat_grid_block(v, s_red);
-    const LatTable g = lat_table_of(v, tab_cap, tsz32);
-    if (g.ok) {  // centres to grid indices, the table, this position's grid indices
-      tw = g.wx;
-      const int ax0 = v[2], ay0 = v[4];  // smallest offsets: index 0 of each axis
+    lat_grid_block(h, s_red);
+    LatCodes cxd = lat_codes(v[0], v[2], v[3], h[2] != h[3]);
+    LatCodes cyd = lat_codes(v[1], v[4], v[5], h[4] != h[5]);
+    if (lat_codes_fit(cxd, cyd, tsz32)) {
+      if ((int64_t)cxd.width * cyd.width <= tab_cap) {
+        tw = cxd.width;
+      } else {  // one step for both axes
+        const int g = (int)gcd_u32((unsigned)v[0], (unsigned)v[1]);
+        const bool half = h[2] != h[3] || h[4] != h[5];
+        cxd = lat_codes(g, v[2], v[3], half);
+        cyd = lat_codes(g, v[4], v[5], half);
+        const int64_t e = max(cxd.width, cyd.width);
+        if (e <= 4096 && e * (e + 1) / 2 <= tab_cap && lat_codes_fit(cxd, cyd, tsz32)) tw = -1;
+      }
+    }
+    if (tw != 0) {
+      const int ox = (o.x >> 1) + v[2], oy = (o.y >> 1) + v[4];
       for (int j = threadIdx.x; j < N; j += blockDim.x)
-        sxy2[j] = make_int2((sxy2[j].x - o.x - ax0) / g.gx, (sxy2[j].y - o.y - ay0) / g.gy);
-      for (int e = threadIdx.x; e < g.wx * g.wy; e += blockDim.x) {
-        const int b = e / g.wx, a = e - b * g.wx;
-        tab[e] = table2[(g.gy * b) * (g.gy * b) + (g.gx * a) * (g.gx * a)];
-      }
-      if (qlat) {
-        QA = ((int)X2 - o.x - ax0) / g.gx;
-        QB = ((int)Y2 - o.y - ay0) / g.gy;
-      }
-      __syncthreads();
-    } else {
-      // The positions on a grid of steps (gx, gy) >= 4 (origin: the block's first
-      // position) and every centre on it or half a pixel (one lattice unit) after it
-      // along each axis (the midpoints of odd window shifts): a centre is at
-      // o + g A + e (e in {0, 1}), an offset p - c = g k - e, so |p - c| is g |k|, g |k| + 1
-      // (e = 1, k <= 0) or g k - 1 (e = 1, k >= 1): the table holds the kernel value of
-      // each (|k|, case) pair per axis, row length jw = 3 Kx.
-      const int q0 = nindices[noff + (int64_t)blockIdx.x * blockDim.x];
-      const double PX2 = 2.0 * px[q0], PY2 = 2.0 * py[q0];
-      const bool oklat = PX2 == rint(PX2) && PY2 == rint(PY2) && fabs(PX2) < 1073741824.0 &&
-                         fabs(PY2) < 1073741824.0;
-      if (oklat) {  // uniform: every thread read the same position
-        const int OX = (int)PX2, OY = (int)PY2;
-        int vp[6];
-        lat_grid_init(vp);
-        if (qlat) lat_grid_add(vp, (int)X2 - OX, (int)Y2 - OY);
-        lat_grid_block(vp, s_red);
-        const int gpx = vp[0], gpy = vp[1];
-        // every position of the block is on the lattice when qlat holds for all of
-        // them: count the others (in the gcd slot, as 0 / 1) with the centres below
-        if (gpx >= 4 && gpy >= 4) {
-          int vc[6];
-          lat_grid_init(vc);
-          vc[0] = (k < M && !qlat) ? 1 : 0;
-          for (int j = threadIdx.x; j < N; j += blockDim.x) {
-            const int dx = sxy2[j].x - OX, dy = sxy2[j].y - OY;
-            const int ax = (dx >= 0) ? dx / gpx : -((-dx + gpx - 1) / gpx);  // floor
-            const int ay = (dy >= 0) ? dy / gpy : -((-dy + gpy - 1) / gpy);
-            const int ex = dx - ax * gpx, ey = dy - ay * gpy;
-            if (ex > 1 || ey > 1) vc[0] = 1;
-            vc[2] = min(vc[2], ax);
-            vc[3] = max(vc[3], ax);
-            vc[4] = min(vc[4], ay);
-            vc[5] = max(vc[5], ay);
+        code[j] = make_int2(cxd.code(code[j].x, ox), cyd.code(code[j].y, oy));
+      Q = make_int2(cxd.code(Q.x, ox), cyd.code(Q.y, oy));
+      if (tw > 0) {
+        for (int e = threadIdx.x; e < cxd.width * cyd.width; e += blockDim.x) {
+          const int b = e / tw, a = e - b * tw;
+          const int dx = cxd.offset(a), dy = cyd.offset(b);
+          tab[e] = table2[dy * dy + dx * dx];
+        }
+      } else {
+        const int wmax = max(cxd.width, cyd.width);
+        for (int a = threadIdx.x >> 5; a < wmax; a += blockDim.x >> 5) {
+          const int da = cxd.offset(a);
+          for (int b = threadIdx.x & 31; b <= a; b += 32) {
+            const int db = cxd.offset(b), kq = da * da + db * db;
+            tab[a * (a + 1) / 2 + b] = kq < tsz32 ? table2[kq] : make_float2(0.f, 0.f);
           }
-          lat_grid_block(vc, s_red);
-          // grid indices of the positions: offsets / g (exact)
-          const int pax0 = vp[2] / gpx, pax1 = vp[3] / gpx, pay0 = vp[4] / gpy,
-                    pay1 = vp[5] / gpy;
-          const int kx = max(pax1 - vc[2], vc[3] - pax0) + 1;
-          const int ky = max(pay1 - vc[4], vc[5] - pay0) + 1;
-          const int64_t ex = (int64_t)gpx * kx + 1, ey = (int64_t)gpy * ky + 1;
-          if (vc[0] == 0 && vc[2] <= vc[3] && kx > 0 && ky > 0 &&
-              (int64_t)9 * kx * ky <= tab_cap && ex <= 32767 && ey <= 32767 &&
-              ex * ex + ey * ey < (int64_t)tsz32) {
-            jw = 3 * kx;
-            for (int j = threadIdx.x; j < N; j += blockDim.x) {
-              const int dx = sxy2[j].x - OX, dy = sxy2[j].y - OY;
-              const int ax = (dx >= 0) ? dx / gpx : -((-dx + gpx - 1) / gpx);
-              const int ay = (dy >= 0) ? dy / gpy : -((-dy + gpy - 1) / gpy);
-              sxy2[j] = make_int2(2 * ax + (dx - ax * gpx), 2 * ay + (dy - ay * gpy));
-            }
-            for (int e = threadIdx.x; e < 9 * kx * ky; e += blockDim.x) {
-              const int r = e / jw, c = e - r * jw;
-              const int axx = c / 3, sx = c - 3 * axx, ayy = r / 3, sy = r - 3 * ayy;
-              const int adx = gpx * axx + (sx == 1 ? 1 : (sx == 2 ? -1 : 0));
-              const int ady = gpy * ayy + (sy == 1 ? 1 : (sy == 2 ? -1 : 0));
-              tab[e] = (adx < 0 || ady < 0) ? make_float2(0.f, 0.f)
-                                            : table2[ady * ady + adx * adx];
-            }
-            if (qlat) {
-              QA = ((int)X2 - OX) / gpx;
-              QB = ((int)Y2 - OY) / gpy;
-            }
-          }
-          __syncthreads();
         }
       }
+      __syncthreads();
     }
   }
   if (k >= M) return;
-  if (qlat && jw > 0) {  // offsets of the jittered grid in the shared table
-    float hx = 0.f, lx = 0.f, hy = 0.f, ly = 0.f;
-    constexpr int U = 8;
-    for (int j0 = 0; j0 < N; j0 += U) {
+  constexpr int U = 8;  // table loads issued ahead of their use
+  float2 hi = make_float2(0.f, 0.f), lo = hi;
+  auto add = [&](float2 f, int j) {
+    const float4 d = dw[j];
+    df_mac_x2(f, make_float2(d.x, d.y), make_float2(d.z, d.w), hi, lo);
+  };
+  // sum over the centres, U at a time, of the table entry at(offset)
+  auto sum = [&](auto at) {
+    int j0 = 0;
+    for (; j0 + U <= N; j0 += U) {
       float2 f[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int2 c = sxy2[min(j0 + u, N - 1)];
-        const int kx = QA - (c.x >> 1), ky = QB - (c.y >> 1);
-        const int sx = (c.x & 1) ? (kx <= 0 ? 1 : 2) : 0;
-        const int sy = (c.y & 1) ? (ky <= 0 ? 1 : 2) : 0;
-        f[u] = tab[(3 * abs(ky) + sy) * jw + 3 * abs(kx) + sx];
-      }
+      for (int u = 0; u < U; ++u) f[u] = at(code[j0 + u]);
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (j0 + u >= N) break;
-        df_mac(dwx[j0 + u], f[u], hx, lx);
-        df_mac(dwy[j0 + u], f[u], hy, ly);
-      }
+      for (int u = 0; u < U; ++u) add(f[u], j0 + u);
     }
-    vx += (double)hx + (double)lx;
-    vy += (double)hy + (double)ly;
-  } else if (qlat && tw > 0) {  // grid offsets in the shared table, double-float sums
-    float hx = 0.f, lx = 0.f, hy = 0.f, ly = 0.f;
-    constexpr int U = 8;
-    for (int j0 = 0; j0 < N; j0 += U) {
-      float2 f[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int2 c = sxy2[min(j0 + u, N - 1)];
-        f[u] = tab[abs(QB - c.y) * tw + abs(QA - c.x)];
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (j0 + u >= N) break;
-        df_mac(dwx[j0 + u], f[u], hx, lx);
-        df_mac(dwy[j0 + u], f[u], hy, ly);
-      }
-    }
-    vx += (double)hx + (double)lx;
-    vy += (double)hy + (double)ly;
+    for (; j0 < N; ++j0) add(at(code[j0]), j0);
+  };
+  if (qlat && tw > 0) {
+    sum([&](int2 c) { return tab[abs(Q.y - c.y) * tw + abs(Q.x - c.x)]; });
+  } else if (qlat && tw < 0) {
+    sum([&](int2 c) {
+      const int dx = abs(Q.x - c.x), dy = abs(Q.y - c.y);
+      const int a = max(dx, dy), b = min(dx, dy);
+      return tab[((a * a + a) >> 1) + b];
+    });
   } else if (qlat && table2 != nullptr) {  // 4 r^2 in integers, double-float sums
-    const int QX = (int)X2, QY = (int)Y2;
-    float hx = 0.f, lx = 0.f, hy = 0.f, ly = 0.f;
-    constexpr int U = 8;  // table loads issued ahead of their use
     for (int j0 = 0; j0 < N; j0 += U) {
       float2 f[U];
       bool far[U];
@@ -1351,8 +1316,8 @@ __global__ void __launch_bounds__(256)
         if (j < N) {
           // 32-bit 4 r^2 (lattice coordinates below 2^30; |dx|, |dy| <= 32767 keeps
           // the sum below 2^31, farther pairs are beyond the table)
-          const int2 c = sxy2[j];
-          const int dx = QX - c.x, dy = QY - c.y;
+          const int2 c = code[j];
+          const int dx = Q.x - c.x, dy = Q.y - c.y;
           const bool near = (unsigned)dx + 32767u <= 65534u && (unsigned)dy + 32767u <= 65534u;
           const int kq = near ? dy * dy + dx * dx : INT_MAX;
           far[u] = kq >= tsz32;
@@ -1368,18 +1333,14 @@ __global__ void __launch_bounds__(256)
           vx = fma(swx[j], fd, vx);
           vy = fma(swy[j], fd, vy);
         } else {
-          df_mac(dwx[j], f[u], hx, lx);
-          df_mac(dwy[j], f[u], hy, ly);
+          add(f[u], j);
         }
       }
     }
-    vx += (double)hx + (double)lx;
-    vy += (double)hy + (double)ly;
   } else if (qlat) {  // 4 r^2 in integer arithmetic, table lookup
-    const int QX = (int)X2, QY = (int)Y2;
     for (int j = 0; j < N; ++j) {
-      const int2 c = sxy2[j];
-      const int64_t dx = (int64_t)(QX - c.x), dy = (int64_t)(QY - c.y);
+      const int2 c = code[j];
+      const int64_t dx = (int64_t)(Q.x - c.x), dy = (int64_t)(Q.y - c.y);
       const int64_t kq = dy * dy + dx * dx;
       const double f = (kq < tsize) ? __ldg(table + kq) : tps_phi(scx[j], scy[j], x, y);
       vx = fma(swx[j], f, vx);
@@ -1392,6 +1353,8 @@ __global__ void __launch_bounds__(256)
       vy = fma(swy[j], f, vy);
     }
   }
+  vx += (double)hi.x + (double)lo.x;
+  vy += (double)hi.y + (double)lo.y;
   vx = fma(swx[N + 2], x, fma(swx[N + 1], y, __dadd_rn(vx, swx[N])));
   vy = fma(swy[N + 2], x, fma(swy[N + 1], y, __dadd_rn(vy, swy[N])));
   const double c = ncoefs[noff + k];
@@ -1695,24 +1658,25 @@ extern "C" int fi_tps_interpolate(const fi_tps_plan* plan, int nb_subdom, int ma
              "fi_tps_interpolate: null pointer");
   FI_REQUIRE(nb_subdom > 0 && npts > 0, "fi_tps_interpolate: bad sizes");
   cudaStream_t s = (cudaStream_t)stream;
-  const size_t base = (size_t)(4 * max_members + 6) * sizeof(double) +
-                      (size_t)max_members * sizeof(int2) +
-                      (size_t)2 * max_members * sizeof(float2);
+  const int nm = (max_members + 4) & ~1;
+  const size_t base = (size_t)nm * (sizeof(float4) + 4 * sizeof(double) + sizeof(int2));
   FI_REQUIRE(base <= 200 * 1024, "fi_tps_interpolate: subdomain of %d vectors too large",
              max_members);
-  // the grid-offset table (at least EVAL_TABLE entries) where it fits beside the
-  // subdomain's centres
   FI_REQUIRE(table_entries >= 0 && table_entries <= 16384,
              "fi_tps_interpolate: table_entries %d out of [0, 16384]", table_entries);
-  const int want = table_entries > EVAL_TABLE ? table_entries : EVAL_TABLE;
+  // the grid-offset table (EVAL_TABLE entries unless the caller asks for its own size) where
+  // it fits beside the subdomain's centres
+  const int want = table_entries > 0 ? table_entries : EVAL_TABLE;
   const int tab_cap = base + (size_t)want * sizeof(float2) <= 200 * 1024 ? want : 0;
   const size_t smem = base + (size_t)tab_cap * sizeof(float2);
   static SmemLimit limit;
   FI_CUDA_TRY(raise_smem_limit(k_tps_eval, smem, limit));
   if (max_new_members > 0) {
-    const int threads = 256;
-    dim3 grid((max_new_members + threads - 1) / threads, nb_subdom);
-    k_tps_eval<<<grid, threads, smem, s>>>(
+    // wide blocks share a large table between more warps; narrow ones where a subdomain's
+    // positions fill few of them
+    const int nt = (int64_t)nb_subdom * (max_new_members / EVAL_NT) >= 152 ? EVAL_NT : 256;
+    dim3 grid((max_new_members + nt - 1) / nt, nb_subdom);
+    k_tps_eval<<<grid, nt, smem, s>>>(
         counts, offsets, indices, w_offsets, weights, cx, cy, ncounts, noffsets, nindices, ncoefs,
         px, py, partx, party, phi_table, reinterpret_cast<const float2*>(phi_table2), table_size,
         cxy2, c_on_lattice, max_members, tab_cap);

@@ -1129,12 +1129,9 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   }
   __syncthreads();
   const bool lat = s_lat != 0;
-  // Centres on the lattice: with x = 2 p + e in half pixels (e = 0, 1) and g the greatest
-  // common divisor of the whole pixels p - p_0 = g a along an axis, an offset of two centres
-  // is 2 g k + s, s = -1, 0, 1 (the window grid, or half a pixel off it where the window
-  // shift was odd).  When the (hi, lo) kernel values of all these offsets fit the panel, cxy
-  // becomes the codes 3 a + e, whose differences 3 k + s index the table (a when every e is
-  // the same, differences k); otherwise it keeps the lattice coordinates.
+  // Centres on the lattice: when the (hi, lo) kernel values of all their offsets fit the
+  // panel, cxy becomes the codes of the centres' grid (lat_codes), whose differences index
+  // the table; otherwise it keeps the lattice coordinates.
   KEntries K{cxy,
              reinterpret_cast<const float2*>(panel + NW * 96 * 2),
              0,
@@ -1144,43 +1141,30 @@ __global__ void __launch_bounds__(NT, 512 / NT)
              yc,
              phi_table,
              table_size};
-  int3 dec_x = make_int3(1, 0, 0), dec_y = dec_x;  // lattice coordinate of a code: see lat_of
+  LatCodes lx{1, 0, false}, ly{1, 0, false};
   if (lat) {
     const int2 o = cxy[0];
-    int v[6], w[6];  // whole pixels; w[2..5]: extremes of the half-pixel parts
+    int v[6], h[6];  // whole pixels; half-pixel parts
     lat_grid_init(v);
-    lat_grid_init(w);
+    lat_grid_init(h);
     for (int i = threadIdx.x; i < N; i += NT) {
       lat_grid_add(v, (cxy[i].x >> 1) - (o.x >> 1), (cxy[i].y >> 1) - (o.y >> 1));
-      lat_grid_add(w, cxy[i].x & 1, cxy[i].y & 1);
+      lat_grid_add(h, cxy[i].x & 1, cxy[i].y & 1);
     }
     lat_grid_block(v, reinterpret_cast<int*>(sh));
-    lat_grid_block(w, reinterpret_cast<int*>(sh));
-    const LatTable g = lat_table_of(v, INT_MAX, INT_MAX);
-    const bool jx = w[2] != w[3], jy = w[4] != w[5];
-    const int64_t wx = jx ? 3 * (int64_t)g.wx - 1 : g.wx, wy = jy ? 3 * (int64_t)g.wy - 1 : g.wy;
-    const int64_t ex = 2 * (int64_t)g.gx * (g.wx - 1) + 1, ey = 2 * (int64_t)g.gy * (g.wy - 1) + 1;
-    if (g.ok && phi_table2 != nullptr && wx * wy <= panel_table(NW) && ex <= 32767 &&
-        ey <= 32767 && ex * ex + ey * ey < (int64_t)K.tsz32) {
-      K.tw = (int)wx;
-      dec_x = make_int3(2 * g.gx, jx, w[2]);
-      dec_y = make_int3(2 * g.gy, jy, w[4]);
-      const int px0 = (o.x >> 1) + v[2], py0 = (o.y >> 1) + v[4];
-      for (int i = threadIdx.x; i < N; i += NT) {
-        const int2 c = cxy[i];
-        const int ax = ((c.x >> 1) - px0) / g.gx, ay = ((c.y >> 1) - py0) / g.gy;
-        cxy[i] = make_int2(jx ? 3 * ax + (c.x & 1) : ax, jy ? 3 * ay + (c.y & 1) : ay);
-      }
-      // offset of a code difference d >= 0: 2 g k + s, d = 3 k + s (or 2 g d)
-      auto offset = [](int d, int3 dec) {
-        if (!dec.y) return dec.x * d;
-        const int k = (d + 1) / 3;
-        return dec.x * k + (d - 3 * k);
-      };
+    lat_grid_block(h, reinterpret_cast<int*>(sh));
+    lx = lat_codes(v[0], v[2], v[3], h[2] != h[3]);
+    ly = lat_codes(v[1], v[4], v[5], h[4] != h[5]);
+    if (phi_table2 != nullptr && (int64_t)lx.width * ly.width <= panel_table(NW) &&
+        lat_codes_fit(lx, ly, K.tsz32)) {
+      K.tw = lx.width;
+      for (int i = threadIdx.x; i < N; i += NT)
+        cxy[i] = make_int2(lx.code(cxy[i].x, (o.x >> 1) + v[2]),
+                           ly.code(cxy[i].y, (o.y >> 1) + v[4]));
       float2* tab = const_cast<float2*>(K.tab);
-      for (int e = threadIdx.x; e < (int)(wx * wy); e += NT) {
-        const int b = e / (int)wx, a = e - b * (int)wx;
-        const int dx = offset(a, dec_x), dy = offset(b, dec_y);
+      for (int e = threadIdx.x; e < lx.width * ly.width; e += NT) {
+        const int b = e / lx.width, a = e - b * lx.width;
+        const int dx = lx.offset(a), dy = ly.offset(b);
         tab[e] = phi_table2[dy * dy + dx * dx];
       }
     }
@@ -1188,13 +1172,12 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   }
   const int kmode = !lat || phi_table2 == nullptr ? K_DIRECT : K.tw > 0 ? K_TABLE : K_GATHER;
   // A = K + lam I, entry (r, c), FP64; on the lattice 4 r^2 is an integer table index
-  auto lat_of = [](int c, int3 dec) { return dec.y ? dec.x * (c / 3) + c % 3 : dec.x * c; };
   auto a_entry = [&](int r, int c) -> double {
     if (r == c) return lam;
     if (lat) {
       const int2 ca = cxy[r], cb = cxy[c];
-      const int64_t dx = lat_of(ca.x, dec_x) - lat_of(cb.x, dec_x);
-      const int64_t dy = lat_of(ca.y, dec_y) - lat_of(cb.y, dec_y);
+      const int64_t dx = K.tw > 0 ? lx.coord(ca.x) - lx.coord(cb.x) : (int64_t)ca.x - cb.x;
+      const int64_t dy = K.tw > 0 ? ly.coord(ca.y) - ly.coord(cb.y) : (int64_t)ca.y - cb.y;
       const int64_t kq = dy * dy + dx * dx;
       if (kq < table_size) return __ldg(phi_table + kq);
       return phi_pair(xc[r], yc[r], xc[c], yc[c], nullptr, 0);

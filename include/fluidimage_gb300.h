@@ -587,7 +587,7 @@ int fi_tps_smooth_fields(const double* px, const double* py, int npts, const flo
  * as nindices.  cxy2/c_on_lattice (nullable, from fi_tps_lattice on the centres)
  * enable integer 4 r^2 table indices; with phi_table2 (nullable, fi_tps_phi_table2)
  * the kernel sums on the lattice run in double-float (~1e-14 relative per term).
- * table_entries (0: 2048, at most 16384): capacity of the per-block shared-memory
+ * table_entries (0: 9216, at most 16384): capacity of the per-block shared-memory
  * copy of the kernel values of a grid's offsets, used where the new positions lie on
  * a grid and the centres on it or half a pixel off it (a larger table costs shared
  * memory, and so L1 capacity, on every block of the launch).
