@@ -97,3 +97,25 @@ def test_griddata_matches_scipy(seed, half, holes, block):
     np.testing.assert_array_equal(ry, np.rint(oy).astype(np.int32))
     # flagged points hold one of the valid values: inside [min, max] of the data
     assert np.all(np.isfinite(ox)) and np.all(np.isfinite(oy))
+
+
+# the smallest sort (nx + ny = 32) and one past it, a large grid with a hole,
+# and steps whose windows leave 13 bits (64-bit predicates at once, and only
+# from a few steps on)
+@pytest.mark.parametrize("nx,ny,step,holes,block", [
+    (16, 16, 16, 0.1, None), (17, 16, 16, 0.1, None), (3, 2, 16, 0.0, None),
+    (150, 140, 8, 0.08, ((60, 66), (70, 75))), (9, 8, 2500, 0.1, None),
+    (14, 13, 1100, 0.2, ((4, 8), (5, 8)))])
+def test_griddata_windows_and_hull_sizes(nx, ny, step, holes, block):
+    c = _case(nx * 1000 + ny, nx=nx, ny=ny, step=step, holes=holes, hole_block=block)
+    ixvecs, iyvecs, cx, cy, sel, vx, vy, qx, qy = c
+    ox, oy, rx, ry, flags, status = _gpu(*c)
+    assert status == 0
+    ok = flags == 0
+    assert ok.mean() > 0.5
+    np.testing.assert_allclose(ox[ok], _scipy(cx, cy, vx.astype(np.float64), qx, qy)[ok],
+                               rtol=0, atol=1e-9)
+    np.testing.assert_allclose(oy[ok], _scipy(cx, cy, vy.astype(np.float64), qx, qy)[ok],
+                               rtol=0, atol=1e-9)
+    np.testing.assert_array_equal(rx, np.rint(ox).astype(np.int32))
+    np.testing.assert_array_equal(ry, np.rint(oy).astype(np.int32))
