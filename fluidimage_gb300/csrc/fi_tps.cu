@@ -146,6 +146,17 @@ __device__ __forceinline__ double f2d_exact(float f) {
   return __longlong_as_double((long long)d);
 }
 
+// Words of the header's 256 bytes that fi_tps_layout uses and leaves zero again.
+struct PlanWords {
+  int ticket;   // blocks done
+  int off[2];   // a centre, a new position off the half-pixel lattice
+};
+__device__ __forceinline__ PlanWords* plan_words(const fi_tps_plan* plan) {
+  return reinterpret_cast<PlanWords*>(
+      reinterpret_cast<unsigned char*>(const_cast<fi_tps_plan*>(plan)) + 128);
+}
+static_assert(sizeof(fi_tps_plan) <= 128, "the words follow the header");
+
 // The plan header from the count of valid vectors and their extremes
 // (ThinPlateSplineSubdom.__init__, thin_plate_spline_subdom.py:38-91).
 __device__ fi_tps_plan plan_header(int base, double xmin, double xmax, double ymin, double ymax,
@@ -261,6 +272,7 @@ __global__ void __launch_bounds__(1024)
   ymax = block_reduce_d(ymax, red, true);
   if (threadIdx.x != 0) return;
   *plan = plan_header(base, xmin, xmax, ymin, ymax, subdom_size, smoothing_coef, pct);
+  *plan_words(plan) = PlanWords{};
 }
 
 // The same compaction over many blocks (large passes), in three launches with the
@@ -374,6 +386,7 @@ __global__ void __launch_bounds__(1024)
     // the float32 extremes are exact in float64 (the positions are float32)
     *plan = plan_header(base, (double)f[0], (double)f[1], (double)f[2], (double)f[3],
                         subdom_size, smoothing_coef, pct);
+    *plan_words(plan) = PlanWords{};
   }
 }
 
@@ -435,18 +448,22 @@ __device__ __forceinline__ int plan_subdoms(const fi_tps_plan* p, int cap) {
   return p->status == 0 ? min(cap, p->nb_subdomx * p->nb_subdomy) : 0;
 }
 
-// count_plan (nullable): the number of points is the plan's centre count (at most npts)
-__global__ void k_tps_lattice(const double* px, const double* py, int npts, int32_t* xy2,
-                              int32_t* on_lattice, const fi_tps_plan* count_plan) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (count_plan != nullptr) npts = plan_centers(count_plan, npts);
-  if (i >= npts) return;
-  const double X = 2.0 * px[i], Y = 2.0 * py[i];
+// (2x, 2y) of a point on the half-pixel lattice, else false and (0, 0)
+__device__ __forceinline__ bool lattice_xy(double x, double y, int2& xy) {
+  const double X = 2.0 * x, Y = 2.0 * y;
   const bool ok = X == rint(X) && Y == rint(Y) && fabs(X) < 1073741824.0 &&
                   fabs(Y) < 1073741824.0;
-  xy2[2 * i] = ok ? (int32_t)X : 0;
-  xy2[2 * i + 1] = ok ? (int32_t)Y : 0;
-  if (!ok) atomicAnd(on_lattice, 0);
+  xy = ok ? make_int2((int)X, (int)Y) : make_int2(0, 0);
+  return ok;
+}
+__global__ void k_tps_lattice(const double* px, const double* py, int npts, int32_t* xy2,
+                              int32_t* on_lattice) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= npts) return;
+  int2 c;
+  if (!lattice_xy(px[i], py[i], c)) atomicAnd(on_lattice, 0);
+  xy2[2 * i] = c.x;
+  xy2[2 * i + 1] = c.y;
 }
 
 __global__ void k_set_int(int32_t* p, int32_t v) { *p = v; }
@@ -456,6 +473,9 @@ __global__ void k_set_int(int32_t* p, int32_t v) { *p = v; }
 // [lo, hi) can only hold points of tiles [first j with tile_pmax[j] >= lo, first j
 // with tile_smin[j] >= hi).
 constexpr int YB_TILE = 256;
+// Up to this many tiles the membership kernels look at all of them and need no running
+// extremes: two loads a thread at 2048 tiles, against a scan launch of 3 us.
+constexpr int YB_SCAN = 2048;
 // Order-preserving 64-bit keys of doubles (NaN excluded): max / min of doubles as
 // integer max / min on the ALU pipe (FP64 is narrow on this GPU).
 __device__ __forceinline__ unsigned long long dkey(double d) {
@@ -472,15 +492,10 @@ __device__ __forceinline__ unsigned long long umin64(unsigned long long a, unsig
   return a < b ? a : b;
 }
 
-__global__ void __launch_bounds__(YB_TILE) k_y_tiles(const double* py, int n, double* tmax,
-                                                      double* tmin,
-                                                      const fi_tps_plan* count_plan) {
+// a block's extremes of y (NaN left out)
+__device__ __forceinline__ void tile_extremes(double y, double* tmax, double* tmin) {
   __shared__ unsigned long long smx[YB_TILE / 32], smn[YB_TILE / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  // with count_plan, n is the plan's centre count; tiles past it stay neutral
-  if (count_plan != nullptr) n = plan_centers(count_plan, n);
-  const int i = blockIdx.x * YB_TILE + threadIdx.x;
-  const double y = (i < n) ? py[i] : NAN;
   unsigned long long kx = isnan(y) ? dkey(-INFINITY) : dkey(y);
   unsigned long long kn = isnan(y) ? dkey(INFINITY) : dkey(y);
   for (int o = 16; o > 0; o >>= 1) {
@@ -497,8 +512,54 @@ __global__ void __launch_bounds__(YB_TILE) k_y_tiles(const double* py, int n, do
       kx = umax64(kx, smx[w]);
       kn = umin64(kn, smn[w]);
     }
-    tmax[blockIdx.x] = dkey_inv(kx);
-    tmin[blockIdx.x] = dkey_inv(kn);
+    *tmax = dkey_inv(kx);
+    *tmin = dkey_inv(kn);
+  }
+}
+__global__ void __launch_bounds__(YB_TILE) k_y_tiles(const double* py, int n, double* tmax,
+                                                      double* tmin) {
+  const int i = blockIdx.x * YB_TILE + threadIdx.x;
+  tile_extremes(i < n ? py[i] : NAN, tmax + blockIdx.x, tmin + blockIdx.x);
+}
+
+// One pass over the centres and the new positions (a block a tile, the centres' tiles
+// first): their half-lattice coordinates and flags (the positions' only if pxy2) and
+// their tiles' extremes.  The last block sets the flags, so that one launch does what a
+// launch each for the flags, the coordinates and the extremes did (2 to 4 us each, all
+// latency).
+__global__ void __launch_bounds__(YB_TILE)
+    k_layout_points(const fi_tps_plan* plan, const double* cx, const double* cy, int ncap,
+                    int ctiles, int32_t* cxy2, int32_t* clat, double* cb, const double* px,
+                    const double* py, int npts, int ptiles, int32_t* pxy2, int32_t* plat,
+                    double* pb) {
+  const int set = (int)blockIdx.x < ctiles ? 0 : 1;
+  const int tile = blockIdx.x - (set == 0 ? 0 : ctiles);
+  const int n = set == 0 ? plan_centers(plan, ncap) : npts;
+  const double* xs = set == 0 ? cx : px;
+  const double* ys = set == 0 ? cy : py;
+  int32_t* xy2 = set == 0 ? cxy2 : pxy2;
+  double* bounds = set == 0 ? cb : pb;
+  const int i = tile * YB_TILE + threadIdx.x;
+  const double y = i < n ? ys[i] : NAN;
+  bool off = false;
+  if (xy2 != nullptr && i < n) {
+    int2 c;
+    off = !lattice_xy(xs[i], y, c);
+    reinterpret_cast<int2*>(xy2)[i] = c;
+  }
+  const bool any_off = __syncthreads_or(off) != 0;
+  tile_extremes(y, bounds + tile, bounds + (set == 0 ? ctiles : ptiles) + tile);
+  if (threadIdx.x == 0) {
+    PlanWords* w = plan_words(plan);
+    if (any_off) atomicOr(&w->off[set], 1);
+    __threadfence();
+    if (atomicAdd(&w->ticket, 1) == (int)gridDim.x - 1) {
+      __threadfence();
+      *clat = atomicExch(&w->off[0], 0) == 0;
+      const int poff = atomicExch(&w->off[1], 0);
+      if (pxy2 != nullptr) *plat = poff == 0;
+      w->ticket = 0;
+    }
   }
 }
 
@@ -692,26 +753,48 @@ __device__ __forceinline__ double coef_norm_hoisted(const double* c, double x, d
   return __dadd_rn(__dmul_rn(__dsub_rn(1.0, dx2), __dsub_rn(1.0, dy2)), 0.001);
 }
 
-// Ordered membership of points in subdomain blockIdx.x; mode 0 counts, mode 1 fills.
-// With the tile index y_pmax / y_smin of py (k_y_tiles) only the tiles that can hold
-// the subdomain's y band are scanned.  subdoms_from_plan: the grid is a capacity,
-// blocks past the plan's subdomains return; centres_from_plan: the points are the
-// plan's centres (npts a capacity).
+// Ordered membership of points in subdomain blockIdx.x, counted or (FILL) listed; TWO:
+// blockIdx.y is the set, so that the centres' and the new positions' counts are one
+// launch (12 us for 7 + 10; the fills are launched apart: with both sets' pointers in
+// registers instead of the constant bank they took 82 us for 26 + 26).  Only the tiles of
+// tmax / tmin (their extremes, or the running ones of fi_tps_y_bounds; null: all) that
+// can hold the subdomain's y band are scanned.  subdoms_from_plan: the grid is a
+// capacity, blocks past the plan's subdomains return.
+struct MemberSet {
+  const double* px;
+  const double* py;
+  int npts;
+  int centres_from_plan;  // the points are the plan's centres (npts a capacity)
+  const int32_t* xy2;
+  const int32_t* on_lattice;
+  const double* tmax;
+  const double* tmin;
+  int32_t* counts;         // counted
+  const int64_t* offsets;  // or filled
+  int32_t* indices;
+  double* coefs;
+};
 constexpr int MEMBER_AXIS = 1024;  // half pixels of a subdomain along an axis
+template <bool FILL, bool TWO>
 __global__ void __launch_bounds__(512)
-    k_tps_members(const fi_tps_plan* plan_ptr, const double* px, const double* py, int npts,
-                  int mode, int32_t* counts, const int64_t* offsets, int32_t* indices,
-                  double* coefs, const int32_t* xy2, const int32_t* on_lattice,
-                  const double* y_pmax, const double* y_smin, int subdoms_from_plan,
-                  int centres_from_plan) {
+    k_tps_members(const fi_tps_plan* plan_ptr, const MemberSet m0, const MemberSet m1,
+                  int subdoms_from_plan) {
   if (subdoms_from_plan && (int)blockIdx.x >= plan_subdoms(plan_ptr, gridDim.x)) return;
-  if (centres_from_plan) npts = plan_centers(plan_ptr, npts);
+  MemberSet m = m0;
+  if (TWO && blockIdx.y != 0) m = m1;
+  const double* const px = m.px;
+  const double* const py = m.py;
+  const int32_t* const xy2 = m.xy2;
+  const int npts = m.centres_from_plan ? plan_centers(plan_ptr, m.npts) : m.npts;
   __shared__ int warp_tot[33];
   __shared__ int s_range[2], s_box[4];
   __shared__ Limits sL;
   __shared__ double s_cn[4];  // coef_norm's subdomain constants: xc, yc, dxm^2, dym^2
   const int i = blockIdx.x;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int nt = (npts + YB_TILE - 1) / YB_TILE;
+  const bool tiled = m.tmax != nullptr && m.tmin != nullptr;
+  const bool look = tiled && nt <= YB_SCAN;
   // the subdomain's limits once per block (FP64 is narrow on this GPU)
   if (threadIdx.x == 0) {
     const fi_tps_plan p = *plan_ptr;
@@ -724,41 +807,58 @@ __global__ void __launch_bounds__(512)
     s_box[1] = (int)fmin(ceil(2.0 * L.lmaxx), kmax);
     s_box[2] = (int)fmin(ceil(2.0 * L.lminy), kmax);
     s_box[3] = (int)fmin(ceil(2.0 * L.lmaxy), kmax);
-    const double xc = __dmul_rn(0.5, __dadd_rn(L.lminx, L.lmaxx));
-    const double yc = __dmul_rn(0.5, __dadd_rn(L.lminy, L.lmaxy));
-    const double dxm = __dsub_rn(L.lmaxx, xc), dym = __dsub_rn(L.lmaxy, yc);
-    s_cn[0] = xc;
-    s_cn[1] = yc;
-    s_cn[2] = __dmul_rn(dxm, dxm);
-    s_cn[3] = __dmul_rn(dym, dym);
+    if (FILL) {
+      const double xc = __dmul_rn(0.5, __dadd_rn(L.lminx, L.lmaxx));
+      const double yc = __dmul_rn(0.5, __dadd_rn(L.lminy, L.lmaxy));
+      const double dxm = __dsub_rn(L.lmaxx, xc), dym = __dsub_rn(L.lmaxy, yc);
+      s_cn[0] = xc;
+      s_cn[1] = yc;
+      s_cn[2] = __dmul_rn(dxm, dxm);
+      s_cn[3] = __dmul_rn(dym, dym);
+    }
     warp_tot[32] = 0;
+    s_range[0] = look ? nt : 0;
+    s_range[1] = look ? 0 : nt;
   }
   __syncthreads();
   const Limits L = sL;
-  // the scanned band: tiles that can hold the subdomain's y range (32-ary searches
-  // by warp 0 over the non-decreasing tile bounds: two rounds of loads for 8k tiles)
-  if (wid == 0) {
-    int q0 = 0, q1 = npts;
-    if (y_pmax != nullptr && y_smin != nullptr) {
-      const int nt = (npts + YB_TILE - 1) / YB_TILE;
-      q0 = min(npts, YB_TILE * warp_lower_bound_ge(y_pmax, nt, L.lminy, lane));
-      q1 = max(q0, min(npts, YB_TILE * warp_lower_bound_ge(y_smin, nt, L.lmaxy, lane)));
+  // the scanned band: tiles that can hold the subdomain's y range, from the first whose
+  // largest y reaches it to the last whose smallest does
+  if (look) {
+    // (integer keys; -0.0 and 0.0 are one value)
+    const unsigned long long klo = dkey(L.lminy == 0.0 ? -0.0 : L.lminy), khi = dkey(L.lmaxy);
+    int first = nt, last = 0;
+    for (int t = threadIdx.x; t < nt; t += blockDim.x) {
+      if (dkey(m.tmax[t]) >= klo) first = min(first, t);
+      if (dkey(m.tmin[t]) < khi) last = t + 1;
     }
+    first = __reduce_min_sync(0xffffffffu, first);
+    last = __reduce_max_sync(0xffffffffu, last);
     if (lane == 0) {
-      s_range[0] = q0;
-      s_range[1] = q1;
+      if (first < nt) atomicMin(&s_range[0], first);
+      if (last > 0) atomicMax(&s_range[1], last);
+    }
+  } else if (tiled && wid == 0) {
+    // running extremes: 32-ary searches (two rounds of loads for 8k tiles)
+    const int t0 = warp_lower_bound_ge(m.tmax, nt, L.lminy, lane);
+    const int t1 = warp_lower_bound_ge(m.tmin, nt, L.lmaxy, lane);
+    if (lane == 0) {
+      s_range[0] = t0;
+      s_range[1] = t1;
     }
   }
-  const bool lat = xy2 != nullptr && on_lattice != nullptr && *on_lattice != 0;
+  const bool lat = xy2 != nullptr && m.on_lattice != nullptr && *m.on_lattice != 0;
   __syncthreads();
   const int X0 = s_box[0], X1 = s_box[1], Y0 = s_box[2], Y1 = s_box[3];
-  const int qb = s_range[0], qe = s_range[1];
-  if (mode == 0) {  // counts only: per-thread tallies, one block reduction
+  const int qb = min(npts, YB_TILE * s_range[0]);
+  const int qe = max(qb, min(npts, YB_TILE * s_range[1]));
+  if (!FILL) {  // per-thread tallies, one block reduction
     int cnt = 0;
+#pragma unroll 4
     for (int q = qb + threadIdx.x; q < qe; q += blockDim.x) {
       if (lat) {
-        const int X = xy2[2 * q], Y = xy2[2 * q + 1];
-        cnt += (X >= X0 && X < X1 && Y >= Y0 && Y < Y1) ? 1 : 0;
+        const int2 XY = reinterpret_cast<const int2*>(xy2)[q];
+        cnt += (XY.x >= X0 && XY.x < X1 && XY.y >= Y0 && XY.y < Y1) ? 1 : 0;
       } else {
         cnt += inside(L, px[q], py[q]) ? 1 : 0;
       }
@@ -766,7 +866,7 @@ __global__ void __launch_bounds__(512)
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if ((threadIdx.x & 31) == 0) atomicAdd(&warp_tot[32], cnt);
     __syncthreads();
-    if (threadIdx.x == 0) counts[i] = warp_tot[32];
+    if (threadIdx.x == 0) m.counts[i] = warp_tot[32];
     return;
   }
   // fill: the band in one contiguous segment per warp; the warps count their members,
@@ -811,7 +911,7 @@ __global__ void __launch_bounds__(512)
     }
     __syncthreads();
   }
-  int64_t pos = offsets[i] + warp_tot[wid];
+  int64_t pos = m.offsets[i] + warp_tot[wid];
   constexpr int R = 4;  // membership of four chunks of 32 tested (loads issued) first
   for (int c0 = s0; c0 < s1; c0 += R * 32) {
     bool in[R];
@@ -826,12 +926,12 @@ __global__ void __launch_bounds__(512)
       const unsigned b = __ballot_sync(0xffffffffu, in[r]);
       if (in[r]) {
         const int64_t at = pos + __popc(b & ((1u << lane) - 1u));
-        indices[at] = q;
+        m.indices[at] = q;
         if (tab) {
           const int2 XY = reinterpret_cast<const int2*>(xy2)[q];
-          coefs[at] = __dadd_rn(__dmul_rn(fac[0][XY.x - X0], fac[1][XY.y - Y0]), 0.001);
+          m.coefs[at] = __dadd_rn(__dmul_rn(fac[0][XY.x - X0], fac[1][XY.y - Y0]), 0.001);
         } else {
-          coefs[at] = coef_norm_hoisted(s_cn, px[q], py[q]);
+          m.coefs[at] = coef_norm_hoisted(s_cn, px[q], py[q]);
         }
       }
       pos += __popc(b);
@@ -1120,6 +1220,48 @@ __device__ __forceinline__ bool on_half_lattice(double v, int& V) {
   return (double)V == t;
 }
 
+// Calls f(member position) for the subdomains of [xr) x [yr) that hold point q, row by
+// row: the place of q in a subdomain's sorted list is a chain of dependent loads, so
+// those of four subdomains are searched together.
+template <typename F>
+__device__ __forceinline__ void for_memberships(int2 xr, int2 yr, int nbx, const int32_t* counts,
+                                                const int64_t* offsets, const int32_t* indices,
+                                                int q, F f) {
+  const int w = xr.y - xr.x, n = max(w, 0) * max(yr.y - yr.x, 0);
+  for (int t0 = 0; t0 < n; t0 += 4) {
+    const int32_t* list[4];
+    int64_t off[4];
+    int lo[4], hi[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      lo[k] = hi[k] = 0;
+      off[k] = 0;
+      if (t0 + k < n) {
+        const int sd = (yr.x + (t0 + k) / w) * nbx + xr.x + (t0 + k) % w;
+        off[k] = offsets[sd];
+        hi[k] = counts[sd] - 1;
+      }
+      list[k] = indices + off[k];
+    }
+    while (lo[0] < hi[0] || lo[1] < hi[1] || lo[2] < hi[2] || lo[3] < hi[3]) {
+      int v[4], mid[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        mid[k] = (lo[k] + hi[k]) >> 1;
+        v[k] = lo[k] < hi[k] ? list[k][mid[k]] : 0;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (lo[k] < hi[k]) {
+          if (v[k] < q) lo[k] = mid[k] + 1; else hi[k] = mid[k];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (t0 + k < n) f(off[k] + lo[k]);
+  }
+}
+
 // Smoothed values at the centres: sum over containing subdomains, in order.
 __global__ void k_tps_blend_centers(const fi_tps_plan* plan_ptr, const double* cx,
                                     const double* cy, const int32_t* counts,
@@ -1139,20 +1281,12 @@ __global__ void k_tps_blend_centers(const fi_tps_plan* plan_ptr, const double* c
   const int2 rx_ = axis_range(bx, x, lat, X);
   const int2 ry_ = axis_range(by, y, lat, Y);
   double sx = 0.0, sy = 0.0, nrm = 0.0;
-  for (int iy = ry_.x; iy < ry_.y; ++iy)
-    for (int ix = rx_.x; ix < rx_.y; ++ix) {
-      const int sd = iy * p.nb_subdomx + ix;
-      const int64_t off = offsets[sd];
-      int lo = 0, hi = counts[sd] - 1;
-      while (lo < hi) {  // members are sorted: find q
-        const int mid = (lo + hi) >> 1;
-        if (indices[off + mid] < q) lo = mid + 1; else hi = mid;
-      }
-      const double c = coefs[off + lo];
-      sx = __dadd_rn(sx, __dmul_rn(c, smx[off + lo]));
-      sy = __dadd_rn(sy, __dmul_rn(c, smy[off + lo]));
-      nrm = __dadd_rn(nrm, c);
-    }
+  for_memberships(rx_, ry_, p.nb_subdomx, counts, offsets, indices, q, [&](int64_t at) {
+    const double c = coefs[at];
+    sx = __dadd_rn(sx, __dmul_rn(c, smx[at]));
+    sy = __dadd_rn(sy, __dmul_rn(c, smy[at]));
+    nrm = __dadd_rn(nrm, c);
+  });
   outx[q] = __ddiv_rn(sx, nrm);
   outy[q] = __ddiv_rn(sy, nrm);
 }
@@ -1380,19 +1514,11 @@ __global__ void k_tps_gather(const fi_tps_plan* plan_ptr, const int32_t* ncounts
   const int2 rx_ = axis_range(bx, x, lat, X);
   const int2 ry_ = axis_range(by, y, lat, Y);
   double sx = 0.0, sy = 0.0, nrm = 0.0;
-  for (int iy = ry_.x; iy < ry_.y; ++iy)
-    for (int ix = rx_.x; ix < rx_.y; ++ix) {
-      const int sd = iy * p.nb_subdomx + ix;
-      const int64_t off = noffsets[sd];
-      int lo = 0, hi = ncounts[sd] - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (nindices[off + mid] < q) lo = mid + 1; else hi = mid;
-      }
-      sx = __dadd_rn(sx, partx[off + lo]);
-      sy = __dadd_rn(sy, party[off + lo]);
-      nrm = __dadd_rn(nrm, ncoefs[off + lo]);
-    }
+  for_memberships(rx_, ry_, p.nb_subdomx, ncounts, noffsets, nindices, q, [&](int64_t at) {
+    sx = __dadd_rn(sx, partx[at]);
+    sy = __dadd_rn(sy, party[at]);
+    nrm = __dadd_rn(nrm, ncoefs[at]);
+  });
   const double vx = __ddiv_rn(sx, nrm), vy = __ddiv_rn(sy, nrm);
   outx[q] = vx;
   outy[q] = vy;
@@ -1432,7 +1558,7 @@ extern "C" int fi_tps_lattice(const double* px, const double* py, int npts, int3
   FI_REQUIRE(px && py && xy2 && on_lattice && npts > 0, "fi_tps_lattice: bad arguments");
   cudaStream_t s = (cudaStream_t)stream;
   k_set_int<<<1, 1, 0, s>>>(on_lattice, 1);
-  k_tps_lattice<<<(npts + 255) / 256, 256, 0, s>>>(px, py, npts, xy2, on_lattice, nullptr);
+  k_tps_lattice<<<(npts + 255) / 256, 256, 0, s>>>(px, py, npts, xy2, on_lattice);
   return check_launch("fi_tps_lattice", 2);
 }
 
@@ -1440,7 +1566,7 @@ extern "C" int fi_tps_y_bounds(const double* py, int npts, double* y_pmax, doubl
                                void* stream) {
   FI_REQUIRE(py && y_pmax && y_smin && npts > 0, "fi_tps_y_bounds: bad arguments");
   const int nt = (npts + YB_TILE - 1) / YB_TILE;
-  k_y_tiles<<<nt, YB_TILE, 0, (cudaStream_t)stream>>>(py, npts, y_pmax, y_smin, nullptr);
+  k_y_tiles<<<nt, YB_TILE, 0, (cudaStream_t)stream>>>(py, npts, y_pmax, y_smin);
   k_y_tiles_scan<<<1, 1024, 0, (cudaStream_t)stream>>>(nt, y_pmax, y_smin);
   return check_launch("fi_tps_y_bounds", 2);
 }
@@ -1467,9 +1593,12 @@ extern "C" int fi_tps_members(const fi_tps_plan* plan, int nb_subdom, const doub
   FI_REQUIRE(mode == 0 ? counts != nullptr : (offsets && indices && coefs),
              "fi_tps_members: missing outputs");
   FI_REQUIRE(((uintptr_t)xy2 & 7) == 0, "fi_tps_members: xy2 must be 8-byte aligned");
-  k_tps_members<<<nb_subdom, 512, 0, (cudaStream_t)stream>>>(plan, px, py, npts, mode, counts,
-                                                            offsets, indices, coefs, xy2,
-                                                            on_lattice, y_pmax, y_smin, 0, 0);
+  const MemberSet set{px, py, npts, 0, xy2, on_lattice, y_pmax, y_smin, counts, offsets,
+                      indices, coefs};
+  if (mode == 0)
+    k_tps_members<false, false><<<nb_subdom, 512, 0, (cudaStream_t)stream>>>(plan, set, set, 0);
+  else
+    k_tps_members<true, false><<<nb_subdom, 512, 0, (cudaStream_t)stream>>>(plan, set, set, 0);
   return check_launch("fi_tps_members");
 }
 
@@ -1489,26 +1618,23 @@ extern "C" int fi_tps_layout(const fi_tps_plan* plan, int nb_subdom, const doubl
   cudaStream_t s = (cudaStream_t)stream;
   const int ctiles = (num_centers + YB_TILE - 1) / YB_TILE;
   const int ptiles = (npts + YB_TILE - 1) / YB_TILE;
-  k_set_int<<<1, 1, 0, s>>>(clat, 1);
-  k_tps_lattice<<<ctiles, 256, 0, s>>>(cx, cy, num_centers, cxy2, clat, plan);
-  int launched = 2;
-  if (!p_given) {
-    k_set_int<<<1, 1, 0, s>>>(plat, 1);
-    k_tps_lattice<<<ptiles, 256, 0, s>>>(px, py, npts, pxy2, plat, nullptr);
+  k_layout_points<<<ctiles + ptiles, YB_TILE, 0, s>>>(
+      plan, cx, cy, num_centers, ctiles, cxy2, clat, cbounds, px, py, npts, ptiles,
+      p_given ? nullptr : pxy2, plat, pbounds);
+  int launched = 3;
+  if (ctiles > YB_SCAN || ptiles > YB_SCAN) {
+    k_y_tiles_scan<<<1, 1024, 0, s>>>(ctiles, cbounds, cbounds + ctiles);
+    k_y_tiles_scan<<<1, 1024, 0, s>>>(ptiles, pbounds, pbounds + ptiles);
     launched += 2;
   }
-  k_y_tiles<<<ctiles, YB_TILE, 0, s>>>(cy, num_centers, cbounds, cbounds + ctiles, plan);
-  k_y_tiles_scan<<<1, 1024, 0, s>>>(ctiles, cbounds, cbounds + ctiles);
-  k_y_tiles<<<ptiles, YB_TILE, 0, s>>>(py, npts, pbounds, pbounds + ptiles, nullptr);
-  k_y_tiles_scan<<<1, 1024, 0, s>>>(ptiles, pbounds, pbounds + ptiles);
-  k_tps_members<<<nb_subdom, 512, 0, s>>>(plan, cx, cy, num_centers, 0, counts, nullptr, nullptr,
-                                          nullptr, cxy2, clat, cbounds, cbounds + ctiles, 1, 1);
-  k_tps_members<<<nb_subdom, 512, 0, s>>>(plan, px, py, npts, 0, ncounts, nullptr, nullptr,
-                                          nullptr, pxy2, plat, pbounds, pbounds + ptiles, 1, 0);
+  k_tps_members<false, true><<<dim3(nb_subdom, 2), 512, 0, s>>>(
+      plan,
+      MemberSet{cx, cy, num_centers, 1, cxy2, clat, cbounds, cbounds + ctiles, counts},
+      MemberSet{px, py, npts, 0, pxy2, plat, pbounds, pbounds + ptiles, ncounts}, 1);
   k_tps_offsets<<<1, 1024, 0, s>>>(counts, ncounts, nb_subdom, offsets, offsets + nb_subdom,
                                    offsets + 2 * nb_subdom, offsets + 3 * nb_subdom,
                                    offsets + 4 * nb_subdom, order, plan);
-  return check_launch("fi_tps_layout", launched + 7);
+  return check_launch("fi_tps_layout", launched);
 }
 
 extern "C" int fi_tps_members_fill(const fi_tps_plan* plan, int nb_subdom, const double* cx,
@@ -1528,12 +1654,12 @@ extern "C" int fi_tps_members_fill(const fi_tps_plan* plan, int nb_subdom, const
   cudaStream_t s = (cudaStream_t)stream;
   const int ctiles = (num_centers + YB_TILE - 1) / YB_TILE;
   const int ptiles = (npts + YB_TILE - 1) / YB_TILE;
-  k_tps_members<<<nb_subdom, 512, 0, s>>>(plan, cx, cy, num_centers, 1, nullptr, offsets,
-                                          indices, coefs, cxy2, clat, cbounds, cbounds + ctiles,
-                                          1, 1);
-  k_tps_members<<<nb_subdom, 512, 0, s>>>(plan, px, py, npts, 1, nullptr, offsets + nb_subdom,
-                                          nindices, ncoefs, pxy2, plat, pbounds,
-                                          pbounds + ptiles, 1, 0);
+  const MemberSet centres{cx, cy, num_centers, 1, cxy2, clat, cbounds, cbounds + ctiles,
+                          nullptr, offsets, indices, coefs};
+  const MemberSet news{px, py, npts, 0, pxy2, plat, pbounds, pbounds + ptiles, nullptr,
+                       offsets + nb_subdom, nindices, ncoefs};
+  k_tps_members<true, false><<<nb_subdom, 512, 0, s>>>(plan, centres, centres, 1);
+  k_tps_members<true, false><<<nb_subdom, 512, 0, s>>>(plan, news, news, 1);
   return check_launch("fi_tps_members_fill", 2);
 }
 

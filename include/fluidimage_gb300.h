@@ -432,7 +432,8 @@ int fi_tps_members(const fi_tps_plan* plan, int nb_subdom, const double* px, con
 /*
  * The layout stages of one TPS interpolation in one call: fi_tps_lattice of the
  * centres (cx, cy) and, unless p_given, of the new positions (px, py) (else pxy2 /
- * plat are read); fi_tps_y_bounds of both; the member counts of both
+ * plat are read); the extremes of y over each 256 of both (running ones, as
+ * fi_tps_y_bounds, beyond 2048 tiles); the member counts of both
  * (fi_tps_members mode 0) and fi_tps_offsets.  nb_subdom and num_centers are
  * capacities (at least the plan's subdomains and valid centres, e.g. nvec for the
  * centres): the kernels read the actual counts from *plan on the device, so that the
@@ -440,12 +441,14 @@ int fi_tps_members(const fi_tps_plan* plan, int nb_subdom, const double* px, con
  * summary after it in one synchronisation; with a plan of more subdomains than
  * nb_subdom, only the first nb_subdom are laid out and the caller calls again with
  * the plan's count.  Buffers: cxy2 [2 num_centers], pxy2 [2 npts], clat / plat [1],
- * cbounds / pbounds [2 ceil(n / 256)] (y_pmax then y_smin, n = num_centers / npts),
+ * cbounds / pbounds [2 ceil(n / 256)] (largest y of each tile, then smallest; n =
+ * num_centers / npts),
  * counts / ncounts [nb_subdom], offsets [4 nb_subdom + 6] (offsets, noffsets,
  * mat_offsets, w_offsets, summary), order (nullable, [nb_subdom]) as in
  * fi_tps_offsets.  No reference counterpart (the
  * bookkeeping of ThinPlateSplineSubdom.__init__ / init_with_new_positions,
- * thin_plate_spline_subdom.py:25-127, 160-206).
+ * thin_plate_spline_subdom.py:25-127, 160-206).  Words after the header in the plan's
+ * FI_TPS_PLAN_BYTES are used meanwhile: one call at a time on a plan.
  */
 int fi_tps_layout(const fi_tps_plan* plan, int nb_subdom, const double* cx, const double* cy,
                   int num_centers, const double* px, const double* py, int npts, int p_given,
