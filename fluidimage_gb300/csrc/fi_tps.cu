@@ -655,6 +655,10 @@ __device__ __forceinline__ int64_t block_scan_i64(int64_t v, int64_t* wsum, int6
 
 // subdomain counts up to which fi_tps_offsets ranks the subdomains by size
 constexpr int ORDER_MAX = 8192;
+// Ranking by counting compares every pair, a sort in shared memory has up to 78 stages:
+// the kernel takes 9.5 and 11.8 us at 342 subdomains, 36 and 14 us at 992.
+constexpr int ORDER_RANK = 512;
+constexpr int ORDER_SORT = 4096;  // (32 KB)
 
 // CSR offsets of the centres' and new positions' membership, offsets of the matrix
 // slots ((n+3)^2 rounded up to 4 elements) and of the weights (2 (n+3)), the
@@ -697,9 +701,10 @@ __global__ void __launch_bounds__(1024)
     summary[4] = s_max[0];
     summary[5] = s_max[1];
   }
-  // solve order: members descending, index ascending among equal counts (stable
-  // rank by counting, O(nsub^2) / 1024 per thread; identity beyond ORDER_MAX)
-  if (order != nullptr) {
+  // solve order: members descending, index ascending among equal counts (identity beyond
+  // ORDER_MAX)
+  if (order == nullptr) return;
+  if (nsub <= ORDER_RANK || nsub > ORDER_SORT) {  // the stable rank by counting
     for (int i = threadIdx.x; i < nsub; i += blockDim.x) {
       int rank = i;
       if (nsub <= ORDER_MAX) {
@@ -712,7 +717,32 @@ __global__ void __launch_bounds__(1024)
       }
       order[rank] = i;
     }
+    return;
   }
+  // bitonic sort of (count, inverted index)
+  __shared__ unsigned long long key[ORDER_SORT];
+  int m = 64;
+  while (m < nsub) m <<= 1;
+  for (int i = threadIdx.x; i < m; i += blockDim.x)
+    key[i] = i < nsub ? ((unsigned long long)(unsigned)counts[i] << 32) | (unsigned)~i : 0ull;
+  __syncthreads();
+  for (int size = 2; size <= m; size <<= 1)
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int j = threadIdx.x; j < m / 2; j += blockDim.x) {
+        const int t = ((j & ~(stride - 1)) << 1) | (j & (stride - 1));
+        const bool down = (t & size) == 0;
+        const unsigned long long x = key[t], y = key[t + stride];
+        if ((x < y) == down) {
+          key[t] = y;
+          key[t + stride] = x;
+        }
+      }
+      // (the pairs of 64 keys stay with one warp)
+      if (stride > 32 || (stride > 1 ? stride >> 1 : size) > 32) __syncthreads();
+      else __syncwarp();
+    }
+  __syncthreads();
+  for (int i = threadIdx.x; i < nsub; i += blockDim.x) order[i] = (int)~(unsigned)key[i];
 }
 
 // First index q in [0, n) with a[q] >= v for a non-decreasing a (n if none).
@@ -776,7 +806,7 @@ struct MemberSet {
 };
 constexpr int MEMBER_AXIS = 1024;  // half pixels of a subdomain along an axis
 template <bool FILL, bool TWO>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(512, FILL ? 3 : 4)
     k_tps_members(const fi_tps_plan* plan_ptr, const MemberSet m0, const MemberSet m1,
                   int subdoms_from_plan) {
   if (subdoms_from_plan && (int)blockIdx.x >= plan_subdoms(plan_ptr, gridDim.x)) return;
@@ -854,14 +884,15 @@ __global__ void __launch_bounds__(512)
   const int qe = max(qb, min(npts, YB_TILE * s_range[1]));
   if (!FILL) {  // per-thread tallies, one block reduction
     int cnt = 0;
+    if (lat) {
 #pragma unroll 4
-    for (int q = qb + threadIdx.x; q < qe; q += blockDim.x) {
-      if (lat) {
+      for (int q = qb + threadIdx.x; q < qe; q += blockDim.x) {
         const int2 XY = reinterpret_cast<const int2*>(xy2)[q];
         cnt += (XY.x >= X0 && XY.x < X1 && XY.y >= Y0 && XY.y < Y1) ? 1 : 0;
-      } else {
-        cnt += inside(L, px[q], py[q]) ? 1 : 0;
       }
+    } else {
+      for (int q = qb + threadIdx.x; q < qe; q += blockDim.x)
+        cnt += inside(L, px[q], py[q]) ? 1 : 0;
     }
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if ((threadIdx.x & 31) == 0) atomicAdd(&warp_tot[32], cnt);
@@ -871,72 +902,76 @@ __global__ void __launch_bounds__(512)
   }
   // fill: the band in one contiguous segment per warp; the warps count their members,
   // one block scan places the segments, then each warp writes its members in order
-  // (ballots within the warp: two barriers in all instead of three per 512 points)
-  auto member = [&](int q) -> bool {
-    if (lat) {
-      const int2 XY = reinterpret_cast<const int2*>(xy2)[q];
-      return XY.x >= X0 && XY.x < X1 && XY.y >= Y0 && XY.y < Y1;
-    }
-    return inside(L, px[q], py[q]);
-  };
-  const int nw = blockDim.x >> 5;
-  const int seg = (((qe - qb) + nw - 1) / nw + 31) & ~31;
-  const int s0 = min(qe, qb + wid * seg), s1 = min(qe, s0 + seg);
-  int cnt = 0;
+  // (ballots within the warp: two barriers in all instead of three per 512 points).
+  // The two tests of membership stay apart: as one, the compiler evaluates both for each
+  // point, and FP64 comparisons are slow (counts of 992 subdomains: 194 us, apart 56)
+  auto fill = [&](auto member) {
+    const int nw = blockDim.x >> 5;
+    const int seg = (((qe - qb) + nw - 1) / nw + 31) & ~31;
+    const int s0 = min(qe, qb + wid * seg), s1 = min(qe, s0 + seg);
+    int cnt = 0;
 #pragma unroll 4
-  for (int q = s0 + lane; q < s1; q += 32) cnt += member(q) ? 1 : 0;
-  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-  if (lane == 0) warp_tot[wid] = cnt;
-  __syncthreads();
-  if (wid == 0) {
-    const int v = lane < nw ? warp_tot[lane] : 0;
-    int incl = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += u;
-    }
-    if (lane < nw) warp_tot[lane] = incl - v;
-  }
-  __syncthreads();
-  // the two factors of coef_norm for every half pixel of the subdomain (the divisions of
-  // every member were bound by the FP64 pipe)
-  __shared__ double fac[2][MEMBER_AXIS];
-  const bool tab = lat && (int64_t)X1 - X0 <= MEMBER_AXIS && (int64_t)Y1 - Y0 <= MEMBER_AXIS;
-  if (tab) {  // 1 - (x - xc)^2 / dxm^2 and the same for y
-    const int wx = max(0, X1 - X0), wy = max(0, Y1 - Y0);
-    for (int t = threadIdx.x; t < wx + wy; t += blockDim.x) {
-      const int ax = t < wx ? 0 : 1, e = t - ax * wx;
-      const double d = __dsub_rn(0.5 * (double)((ax ? Y0 : X0) + e), s_cn[ax]);
-      fac[ax][e] = __dsub_rn(1.0, __ddiv_rn(__dmul_rn(d, d), s_cn[2 + ax]));
+    for (int q = s0 + lane; q < s1; q += 32) cnt += member(q) ? 1 : 0;
+    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    if (lane == 0) warp_tot[wid] = cnt;
+    __syncthreads();
+    if (wid == 0) {
+      const int v = lane < nw ? warp_tot[lane] : 0;
+      int incl = v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+      }
+      if (lane < nw) warp_tot[lane] = incl - v;
     }
     __syncthreads();
-  }
-  int64_t pos = m.offsets[i] + warp_tot[wid];
-  constexpr int R = 4;  // membership of four chunks of 32 tested (loads issued) first
-  for (int c0 = s0; c0 < s1; c0 += R * 32) {
-    bool in[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int q = c0 + 32 * r + lane;
-      in[r] = q < s1 && member(q);
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int q = c0 + 32 * r + lane;
-      const unsigned b = __ballot_sync(0xffffffffu, in[r]);
-      if (in[r]) {
-        const int64_t at = pos + __popc(b & ((1u << lane) - 1u));
-        m.indices[at] = q;
-        if (tab) {
-          const int2 XY = reinterpret_cast<const int2*>(xy2)[q];
-          m.coefs[at] = __dadd_rn(__dmul_rn(fac[0][XY.x - X0], fac[1][XY.y - Y0]), 0.001);
-        } else {
-          m.coefs[at] = coef_norm_hoisted(s_cn, px[q], py[q]);
-        }
+    // the two factors of coef_norm for every half pixel of the subdomain (the divisions of
+    // every member were bound by the FP64 pipe)
+    __shared__ double fac[2][MEMBER_AXIS];
+    const bool tab = lat && (int64_t)X1 - X0 <= MEMBER_AXIS && (int64_t)Y1 - Y0 <= MEMBER_AXIS;
+    if (tab) {  // 1 - (x - xc)^2 / dxm^2 and the same for y
+      const int wx = max(0, X1 - X0), wy = max(0, Y1 - Y0);
+      for (int t = threadIdx.x; t < wx + wy; t += blockDim.x) {
+        const int ax = t < wx ? 0 : 1, e = t - ax * wx;
+        const double d = __dsub_rn(0.5 * (double)((ax ? Y0 : X0) + e), s_cn[ax]);
+        fac[ax][e] = __dsub_rn(1.0, __ddiv_rn(__dmul_rn(d, d), s_cn[2 + ax]));
       }
-      pos += __popc(b);
+      __syncthreads();
     }
-  }
+    int64_t pos = m.offsets[i] + warp_tot[wid];
+    constexpr int R = 4;  // membership of four chunks of 32 tested (loads issued) first
+    for (int c0 = s0; c0 < s1; c0 += R * 32) {
+      bool in[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int q = c0 + 32 * r + lane;
+        in[r] = q < s1 && member(q);
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int q = c0 + 32 * r + lane;
+        const unsigned b = __ballot_sync(0xffffffffu, in[r]);
+        if (in[r]) {
+          const int64_t at = pos + __popc(b & ((1u << lane) - 1u));
+          m.indices[at] = q;
+          if (tab) {
+            const int2 XY = reinterpret_cast<const int2*>(xy2)[q];
+            m.coefs[at] = __dadd_rn(__dmul_rn(fac[0][XY.x - X0], fac[1][XY.y - Y0]), 0.001);
+          } else {
+            m.coefs[at] = coef_norm_hoisted(s_cn, px[q], py[q]);
+          }
+        }
+        pos += __popc(b);
+      }
+    }
+  };
+  if (lat)
+    fill([&](int q) {
+      const int2 XY = reinterpret_cast<const int2*>(xy2)[q];
+      return XY.x >= X0 && XY.x < X1 && XY.y >= Y0 && XY.y < Y1;
+    });
+  else
+    fill([&](int q) { return inside(L, px[q], py[q]); });
 }
 
 // Block argmax of |col[k..n-1]| with the first index on ties (LAPACK idamax).

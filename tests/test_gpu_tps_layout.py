@@ -1,6 +1,6 @@
 """fi_tps_layout and fi_tps_members_fill (both point sets together, the y-band tiles)
 against fi_tps_members over every point, one set at a time: equal counts, members,
-coefficients and flags."""
+coefficients and flags; the solve order against a stable sort of the counts."""
 
 import numpy as np
 import pytest
@@ -8,10 +8,12 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-# one tile; a remainder; more tiles than are looked at directly (running extremes)
+# one tile; a remainder; more tiles than are looked at directly (running extremes); an
+# order by rank, sorted, and by rank past the sort's shared memory
 @pytest.mark.parametrize("ny,nx,shuffled,lattice", [
     (9, 25, False, True), (33, 31, True, False), (70, 90, True, True),
-    (702, 760, False, True), (702, 760, False, False)])
+    (360, 370, True, True), (702, 760, False, True), (702, 760, False, False),
+    (900, 1000, False, True)])
 def test_layout_matches_full_scans(ny, nx, shuffled, lattice):
     import torch
 
@@ -46,15 +48,18 @@ def test_layout_matches_full_scans(ny, nx, shuffled, lattice):
     cxy2, pxy2, clat, plat = new(2 * n, i32), new(2 * n, i32), new(1, i32), new(1, i32)
     cb, pb = new(2 * ct, f64), new(2 * pt, f64)
     counts, ncounts, offs = new(cap, i32), new(cap, i32), new(4 * cap + 6, i64)
+    order = new(cap, i32)
     idx, nidx, co, nco = new(4 * n, i32), new(4 * n, i32), new(4 * n, f64), new(4 * n, f64)
     for _ in range(2):  # twice on one plan
         L.check(lib.fi_tps_layout(p(plan), cap, p(cx), p(cy), n, p(px), p(py), n, 0, p(cxy2),
                                   p(clat), p(pxy2), p(plat), p(cb), p(pb), p(counts), p(ncounts),
-                                  p(offs), None, None), "layout")
+                                  p(offs), p(order), None), "layout")
     L.check(lib.fi_tps_members_fill(p(plan), cap, p(cx), p(cy), n, p(px), p(py), n, p(cxy2),
                                     p(clat), p(pxy2), p(plat), p(cb), p(pb), p(offs), p(idx),
                                     p(co), p(nidx), p(nco), None), "fill")
     torch.cuda.synchronize()
+    want = torch.sort(counts[:nsub], descending=True, stable=True).indices
+    assert torch.equal(order[:nsub], want.to(i32))
     for (qx, qy, k, xy2, lat, cnt, ind, cf, o0) in (
             (cx, cy, nv, cxy2, clat, counts, idx, co, 0),
             (px, py, n, pxy2, plat, ncounts, nidx, nco, cap)):
