@@ -8,8 +8,9 @@
 // exact for every type.  Which kernel runs:
 //   minimum and maximum of 2-D windows: k_minmax_tile (separable, tiles in shared memory)
 //   any rank of a window along time only: k_time_rank (a pixel's frames in shared memory)
-//   other ranks of 2-D windows up to 32 x 32 of 8, 16 and 32 bit types: k_rank_planes
-//   other ranks of larger 2-D windows: k_rank_select_tile while the tile fits
+//   other ranks of 2-D windows up to 32 x 32 of 8, 16 and 32 bit types: k_rank_planes where
+//   planes_pay
+//   other ranks of 2-D windows: k_rank_select_tile while the tile fits
 //   the rest (3-D windows, float64 medians): k_minmax_axis, k_rank_select
 #include <cstdint>
 #include <cstring>
@@ -603,6 +604,26 @@ static bool takes_minmax_tile(int dtype, int st, int sy, int sx, int rank) {
   return st == 1 && is_extreme((int64_t)sy * sx, rank) &&
          minmax_tile_bytes(sy, sx, key_bytes(dtype)) <= MM_MAX_SMEM;
 }
+// k_rank_planes or k_rank_select_tile (both exact).  A thread of the second counts its
+// window's values for every bit: 17.5 ns per value and bit, 0.2 ps per pixel, value and bit
+// once the chip is full.  A warp of the first takes a 32 x 32 tile in a time that hardly
+// depends on the window and not on how many tiles there are while all are resident (16, 8
+// or 4 warps an SM by the planes' size): 70 to 390 us for 8 bits, 260 to 1260 for 16, 1440
+// to 1900 for 32, less for images than for noise and for large windows; the lines lie at
+// the values below.  Median, us, planes and select, particle image / noise:
+//   u8  512^2  5 x 5: 160 and 34 / 343 and 33;      30 x 30: 78 and 476 / 160 and 476
+//   u16 512^2  5 x 5: 563 and 46 / 1208 and 56;     30 x 30: 344 and 703 / 1029 and 934
+//   u16 2048^2 9 x 9: 1355 and 1113 / 3557 and 1458; 30 x 30: 726 and 9212 / 3058 and 12251
+//   f32 1024^2 16 x 16: 3483 and 1754 / 3132 and 1753; 30 x 30: 2763 and 6343 / 3013 and 6341
+static bool planes_pay(int dtype, int nt, int ny, int nx, int sy, int sx) {
+  const int bits = dtype == FI_PRE_U8 ? 8 : dtype == FI_PRE_U16 ? 16 : 32;
+  const double tile_us = bits == 8 ? 180.0 : bits == 16 ? 600.0 : 1700.0;
+  const double resident = 152.0 * 128 / bits;
+  const double tiles = (double)nt * ((ny + RP_T - 1) / RP_T) * ((nx + RP_T - 1) / RP_T);
+  const double counts = (double)sy * sx * bits, pixels = (double)nt * ny * nx;
+  const double select_us = counts * (pixels * 2.03e-7 > 0.0175 ? pixels * 2.03e-7 : 0.0175);
+  return select_us > tile_us * (tiles > resident ? tiles / resident : 1.0);
+}
 static bool takes_time(int dtype, int nt, int st, int sy, int sx) {
   return sy == 1 && sx == 1 && st > 1 &&
          (dtype == FI_PRE_F64 ? time_bytes<uint64_t>(nt, st) : time_bytes<uint32_t>(nt, st)) <=
@@ -710,7 +731,8 @@ static int rank_filter(const void* in, int dtype, int nt, int ny, int nx, int st
     k_keys_out<<<g, 256, 0, s>>>(k0, count, ro);
     return check_launch("fi_rank_filter", 4);
   }
-  if (tiled && st == 1 && dtype != FI_PRE_F64 && sy <= RP_MAX_WINDOW && sx <= RP_MAX_WINDOW) {
+  if (tiled && st == 1 && dtype != FI_PRE_F64 && sy <= RP_MAX_WINDOW && sx <= RP_MAX_WINDOW &&
+      planes_pay(dtype, nt, ny, nx, sy, sx)) {
     if (dtype == FI_PRE_U8)
       return launch_planes<8>(in, dtype, nt, ny, nx, sy, sx, rank, mode, (uint32_t)ckey, ro, s);
     if (dtype == FI_PRE_U16)
