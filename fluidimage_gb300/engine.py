@@ -223,7 +223,8 @@ class TpsOutput:
 #: half-integer lattice (32 MiB per device); larger distances use log() directly.
 PHI_TABLE_SIZE = 1 << 22
 #: entries of the shared table of kernel values that the final TPS evaluation asks
-#: for (9 K^2 for offsets up to K - 1 grid steps: K = 26 covers subdomains of ~25 steps)
+#: for ((3 K - 1)^2 for offsets up to K - 1 grid steps, or the triangle of that square:
+#: K = 26 or 36)
 FINAL_EVAL_TABLE = 6144
 #: largest subdomain handled by the mixed-precision solver (shared-memory bound)
 MP_MAX_MEMBERS = 800

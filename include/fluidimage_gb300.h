@@ -591,9 +591,10 @@ int fi_tps_smooth_fields(const double* px, const double* py, int npts, const flo
  * enable integer 4 r^2 table indices; with phi_table2 (nullable, fi_tps_phi_table2)
  * the kernel sums on the lattice run in double-float (~1e-14 relative per term).
  * table_entries (0: 9216, at most 16384): capacity of the per-block shared-memory
- * copy of the kernel values of a grid's offsets, used where the new positions lie on
- * a grid and the centres on it or half a pixel off it (a larger table costs shared
- * memory, and so L1 capacity, on every block of the launch).
+ * table of the kernel values of a block's offsets (a rectangle, or the triangle of the
+ * larger offset), used where positions and centres lie on one grid, on grids of which one
+ * is finer, or half a pixel off them (a larger table costs shared memory, and so L1
+ * capacity, on every block of the launch).
  */
 int fi_tps_interpolate(const fi_tps_plan* plan, int nb_subdom, int max_members,
                        int max_new_members, const double* cx, const double* cy,
