@@ -62,11 +62,11 @@ def fft_flops(n):
     return 3 * 2.5 * n * n * math.log2(n * n) + 5 * n * n
 
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of k_tps_solve_mp per subdomain:
-# one CTA of 16 warps per subdomain (launches of at most one subdomain per SM; 72
-# subdomains of the config-2 recipe at 1024^2) and two 8-warp CTAs per SM (the
-# 342-subdomain launch of the 2048^2 workload)
-TPS_DRAM_BYTES_PER_SUBDOMAIN_WIDE = (126.285056e6 + 80.334336e6) / 72
-TPS_DRAM_BYTES_PER_SUBDOMAIN_NARROW = (837.309952e6 + 579.323136e6) / 342
+# CTAs of 16 warps (launches of at most one subdomain per SM; the 72 subdomains between
+# the last passes of the 2048^2 workload) and two 8-warp CTAs per SM (its last 342
+# subdomains, in two launches)
+TPS_DRAM_BYTES_PER_SUBDOMAIN_WIDE = (17.109248e6 + 34.920192e6) / 72
+TPS_DRAM_BYTES_PER_SUBDOMAIN_NARROW = (771.367680e6 + 331.378944e6 + 1.211136e6 + 0.166656e6) / 342
 
 
 def parse_args():
