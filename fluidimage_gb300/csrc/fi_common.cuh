@@ -35,11 +35,12 @@ void add_launches(int k);
     }                                                                         \
   } while (0)
 
-// Raises a kernel's dynamic shared-memory limit to at least `bytes` (above the 48 KB
-// default) on the current device, calling the runtime only when the limit has to
-// grow there.  The attribute is per device, so the call site's record keeps the
-// limit set so far for each device, read and written under one mutex so that host
-// threads launching concurrently never lower it.
+// Raises a kernel's dynamic shared-memory limit to at least `bytes` on the current device,
+// calling the runtime only when the limit has to grow there.  Without a call it is 48 KB
+// less the kernel's own (static) shared memory, asked for once.  The attribute is per
+// device, so the call site's record keeps the limit for each device (0: not asked yet),
+// read and written under one mutex so that host threads launching concurrently never
+// lower it.
 inline std::mutex& smem_limit_mutex() {
   static std::mutex m;
   return m;
@@ -50,17 +51,25 @@ struct SmemLimit {
 };
 template <typename Kernel>
 inline cudaError_t raise_smem_limit(Kernel* kernel, size_t bytes, SmemLimit& rec) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
   int dev = 0;
-  const cudaError_t ed = cudaGetDevice(&dev);
-  if (ed != cudaSuccess) return ed;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lock(smem_limit_mutex());
   const bool cached = dev >= 0 && dev < FI_SMEM_DEVICES;
-  if (cached && bytes <= rec.bytes[dev]) return cudaSuccess;
-  const cudaError_t e =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess && cached) rec.bytes[dev] = bytes;
-  return e;
+  size_t limit = cached ? rec.bytes[dev] : 0;
+  if (limit == 0) {
+    cudaFuncAttributes attr;
+    e = cudaFuncGetAttributes(&attr, kernel);
+    if (e != cudaSuccess) return e;
+    limit = 48 * 1024 - attr.sharedSizeBytes;
+  }
+  if (bytes > limit) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    limit = bytes;
+  }
+  if (cached) rec.bytes[dev] = limit;
+  return cudaSuccess;
 }
 
 inline int check_launch(const char* what, int kernels = 1) {
