@@ -602,6 +602,15 @@ __global__ void k_subtract_weighted(const void* img, const void* filt, int64_t c
 }
 
 // ------------------------------------------------------------------ dispatch
+// Whether the arrays of na bytes at a and nb bytes at b share any.
+static bool overlap(const void* a, size_t na, const void* b, size_t nb) {
+  return (uintptr_t)a < (uintptr_t)b + nb && (uintptr_t)b < (uintptr_t)a + na;
+}
+
+static size_t element_bytes(int dtype) {
+  return dtype == FI_PRE_U8 ? 1 : dtype == FI_PRE_U16 ? 2 : dtype == FI_PRE_F32 ? 4 : 8;
+}
+
 static int key_bytes(int dtype) {
   return dtype == FI_PRE_U8 || dtype == FI_PRE_U16 ? 2 : dtype == FI_PRE_F32 ? 4 : 8;
 }
@@ -709,14 +718,19 @@ static int rank_filter(const void* in, int dtype, int nt, int ny, int nx, int st
   // the frames of a stack are a launch dimension (at most 65535) of the tiled kernels, the
   // tile rows of a frame another
   const bool tiled = nt <= 65535 && ny <= 65535 * RS_TY;
-  if (tiled && takes_minmax_tile(dtype, st, sy, sx, rank)) {
+  // minima and maxima whose output overlaps the input: the kernels of one pass would read
+  // what other blocks have written; the axis passes write only after all of it is read
+  const size_t nbytes = count * element_bytes(dtype);
+  const bool in_place = ro.img == nullptr && is_extreme(wsize, rank) &&
+                        overlap(in, nbytes, ro.out, nbytes);
+  if (!in_place && tiled && takes_minmax_tile(dtype, st, sy, sx, rank)) {
     if (key_bytes(dtype) == 2)
       return launch_minmax_tile<uint16_t>(in, dtype, nt, ny, nx, sy, sx, mode, ckey, is_max, ro, s);
     if (key_bytes(dtype) == 4)
       return launch_minmax_tile<uint32_t>(in, dtype, nt, ny, nx, sy, sx, mode, ckey, is_max, ro, s);
     return launch_minmax_tile<uint64_t>(in, dtype, nt, ny, nx, sy, sx, mode, ckey, is_max, ro, s);
   }
-  if (takes_time(dtype, nt, st, sy, sx)) {
+  if (!in_place && takes_time(dtype, nt, st, sy, sx)) {
     const int64_t npix = (int64_t)ny * nx;
     // packed elements: every frame (and output frame) starts on a whole word, the
     // double pairs of the subtraction on 16 bytes
@@ -806,7 +820,9 @@ extern "C" int fi_rank_subtract(const void* in, void* out, int dtype, int nt, in
   if (check_rank_args(in, out, dtype, nt, ny, nx, st, sy, sx, mode) != FI_OK ||
       check_subtract("fi_rank_subtract", dtype, out_dtype) != FI_OK)
     return FI_ERR_INVALID;
-  FI_REQUIRE(out != in, "fi_rank_subtract: the output must not be the input");
+  const size_t count = (size_t)nt * ny * nx;
+  FI_REQUIRE(!overlap(in, count * element_bytes(dtype), out, count * element_bytes(out_dtype)),
+             "fi_rank_subtract: the output overlaps the input");
   const RankOut ro{out, in, dtype, Subtract::make(dtype, weight, out_dtype, clamp)};
   return rank_filter(in, dtype, nt, ny, nx, st, sy, sx, rank, mode, cval, scratch, ro,
                      (cudaStream_t)stream);

@@ -627,7 +627,8 @@ int fi_tps_interpolate(const fi_tps_plan* plan, int nb_subdom, int max_members,
  * (scipy.ndimage.rank_filter semantics: window [i - s//2, i - s//2 + s - 1], the
  * boundary mode and cval); rank 0 / st*sy*sx - 1 are the minimum / maximum filters
  * (scratch: 2 * nt*ny*nx uint64 when fi_rank_needs_scratch, else nullable), other
- * ranks an exact radix select.
+ * ranks an exact radix select.  The output may overlap the input for minima and maxima
+ * only, with the scratch.
  * Replaces ndi.minimum_filter / median_filter / percentile_filter in sliding_* and
  * temporal_* (works/preproc/_toolbox_py.py:66-155, 189-256).
  */
@@ -645,7 +646,7 @@ int fi_subtract_weighted(const void* img, const void* filtered, int dtype, int64
 
 /*
  * The rank filter and the subtraction in one pass: out = in - weight * filtered with
- * the arguments of fi_rank_filter and fi_subtract_weighted (out is not in).
+ * the arguments of fi_rank_filter and fi_subtract_weighted (out must not overlap in).
  */
 int fi_rank_subtract(const void* in, void* out, int dtype, int nt, int ny, int nx, int st, int sy,
                      int sx, int rank, int mode, double cval, double weight, int out_dtype,
