@@ -14,17 +14,6 @@
 
 namespace fi {
 
-static int num_sms() {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 152;
-  }
-  return sms;
-}
-
 // resident blocks per SM asked of the register allocator: about 128 / 170 registers
 // for 24-32 / 48-64 px windows; for 16 px windows two budgets (128 registers with 16
 // windows per block, ~100 with 8) for the tuner to choose from

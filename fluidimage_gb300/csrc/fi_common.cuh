@@ -72,6 +72,17 @@ inline cudaError_t raise_smem_limit(Kernel* kernel, size_t bytes, SmemLimit& rec
   return cudaSuccess;
 }
 
+// SMs of the device that was current at the first call.
+inline int num_sms() {
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n > 0 ? n : 152;
+  }();
+  return sms;
+}
+
 inline int check_launch(const char* what, int kernels = 1) {
   add_launches(kernels);
   cudaError_t e = cudaGetLastError();

@@ -135,17 +135,6 @@ __global__ void k_min_decode(uint32_t* keys) {
   }
 }
 
-static int num_sms() {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 152;
-  }
-  return sms;
-}
-
 template <int N, bool FW>
 static int launch_pass(const fi_piv_pass_args& a, const float* w0, const float* w1, int nvec,
                        int npad, int do_peaks, cudaStream_t s) {
