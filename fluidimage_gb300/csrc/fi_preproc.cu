@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(GS_NT)
     for (int j = 1; j <= radius; ++j)
       acc += (unsigned long long)((unsigned)p[-j * step] + p[j * step]) * wi[j];
     const unsigned long long frac = acc & 0x7fffffffull;
-    if (acc != 0ull && (frac < e || frac + e >= 0x80000000ull || always)) {
+    if (always || (acc != 0ull && (frac < e || frac + e >= 0x80000000ull))) {
       double a = __dmul_rn((double)p[0], gw.w[radius]);
       for (int j = radius; j >= 1; --j)
         a = __dadd_rn(a, __dmul_rn((double)((int)p[-j * step] + (int)p[j * step]), gw.w[radius - j]));
