@@ -159,6 +159,15 @@ struct Subtract {
   }
 };
 
+// Whether the arrays of na bytes at a and nb bytes at b share any.
+static inline bool overlap(const void* a, size_t na, const void* b, size_t nb) {
+  return (uintptr_t)a < (uintptr_t)b + nb && (uintptr_t)b < (uintptr_t)a + na;
+}
+
+static inline size_t element_bytes(int dtype) {
+  return dtype == FI_PRE_U8 ? 1 : dtype == FI_PRE_U16 ? 2 : dtype == FI_PRE_F32 ? 4 : 8;
+}
+
 static inline int grid_for(int64_t count) {
   const int64_t b = (count + 255) / 256;
   return (int)(b < 152 * 16 ? (b > 0 ? b : 1) : 152 * 16);

@@ -816,6 +816,10 @@ extern "C" int fi_sharpen(const void* in, void* out, void* blurred, int dtype, i
              "fi_sharpen: bad sizes");
   FI_REQUIRE(radius1 >= 0 && radius1 <= GS_MAX_RADIUS && radius2 >= 0 && radius2 <= GS_MAX_RADIUS,
              "fi_sharpen: radius above %d", GS_MAX_RADIUS);
+  const size_t nbytes = (size_t)nt * ny * nx * element_bytes(dtype);
+  FI_REQUIRE(!overlap(in, nbytes, blurred, nbytes) &&
+                 !overlap(out, (size_t)nt * ny * nx * sizeof(double), blurred, nbytes),
+             "fi_sharpen: blurred overlaps the input or the output");
   cudaStream_t s = (cudaStream_t)stream;
   int e;
   if (dtype == FI_PRE_U8) {

@@ -607,15 +607,6 @@ __global__ void k_subtract_weighted(const void* img, const void* filt, int64_t c
 }
 
 // ------------------------------------------------------------------ dispatch
-// Whether the arrays of na bytes at a and nb bytes at b share any.
-static bool overlap(const void* a, size_t na, const void* b, size_t nb) {
-  return (uintptr_t)a < (uintptr_t)b + nb && (uintptr_t)b < (uintptr_t)a + na;
-}
-
-static size_t element_bytes(int dtype) {
-  return dtype == FI_PRE_U8 ? 1 : dtype == FI_PRE_U16 ? 2 : dtype == FI_PRE_F32 ? 4 : 8;
-}
-
 static int key_bytes(int dtype) {
   return dtype == FI_PRE_U8 || dtype == FI_PRE_U16 ? 2 : dtype == FI_PRE_F32 ? 4 : 8;
 }

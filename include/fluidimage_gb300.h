@@ -763,7 +763,8 @@ int fi_gaussian_filter(const void* in, void* out, void* tmp, int dtype, int nt, 
  * sharpen of 8 and 16 bit images (_toolbox_py.py:472-490): the gaussian filter with
  * weights1 into blurred, the one with weights2 on it, and the combination of
  * fi_sharpen_combine into out (float64).  The weights (2 radius + 1 doubles each,
- * radius at most 32, symmetric) are host memory, read before the call returns.
+ * radius at most 32, symmetric) are host memory, read before the call returns; blurred
+ * must overlap neither in nor out.
  */
 int fi_sharpen(const void* in, void* out, void* blurred, int dtype, int nt, int ny, int nx,
                const double* weights1, int radius1, const double* weights2, int radius2,

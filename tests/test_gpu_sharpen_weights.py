@@ -41,3 +41,17 @@ def test_any_weights(weights, dtype):
         assert int(b.max()) > 0
         assert torch.equal(blurred, b)
         assert torch.equal(out, want)
+
+
+def test_blurred_apart_from_the_images():
+    import torch
+
+    from fluidimage_gb300 import _lib as L
+
+    store = torch.zeros(64 * 64 * 10, dtype=torch.uint8, device="cuda")
+    w = np.array([0.25, 0.5, 0.25])
+    at = lambda k: L.ptr(store[k * 64 * 64:])  # noqa: E731
+    for x, out, blurred in ((0, 2, 0), (0, 1, 2), (1, 2, 0)):
+        rc = L.load().fi_sharpen(at(x), at(out), at(blurred) + 64, 0, 1, 64, 64, w.ctypes.data, 1,
+                                 w.ctypes.data, 1, 3.0, L.stream_handle())
+        assert rc != 0
