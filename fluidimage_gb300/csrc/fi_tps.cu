@@ -146,17 +146,6 @@ __device__ __forceinline__ double f2d_exact(float f) {
   return __longlong_as_double((long long)d);
 }
 
-// Words of the header's 256 bytes that fi_tps_layout uses and leaves zero again.
-struct PlanWords {
-  int ticket;   // blocks done
-  int off[2];   // a centre, a new position off the half-pixel lattice
-};
-__device__ __forceinline__ PlanWords* plan_words(const fi_tps_plan* plan) {
-  return reinterpret_cast<PlanWords*>(
-      reinterpret_cast<unsigned char*>(const_cast<fi_tps_plan*>(plan)) + 128);
-}
-static_assert(sizeof(fi_tps_plan) <= 128, "the words follow the header");
-
 // The plan header from the count of valid vectors and their extremes
 // (ThinPlateSplineSubdom.__init__, thin_plate_spline_subdom.py:38-91).
 __device__ fi_tps_plan plan_header(int base, double xmin, double xmax, double ymin, double ymax,
@@ -272,7 +261,6 @@ __global__ void __launch_bounds__(1024)
   ymax = block_reduce_d(ymax, red, true);
   if (threadIdx.x != 0) return;
   *plan = plan_header(base, xmin, xmax, ymin, ymax, subdom_size, smoothing_coef, pct);
-  *plan_words(plan) = PlanWords{};
 }
 
 // The same compaction over many blocks (large passes), in three launches with the
@@ -386,7 +374,6 @@ __global__ void __launch_bounds__(1024)
     // the float32 extremes are exact in float64 (the positions are float32)
     *plan = plan_header(base, (double)f[0], (double)f[1], (double)f[2], (double)f[3],
                         subdom_size, smoothing_coef, pct);
-    *plan_words(plan) = PlanWords{};
   }
 }
 
@@ -522,11 +509,19 @@ __global__ void __launch_bounds__(YB_TILE) k_y_tiles(const double* py, int n, do
   tile_extremes(i < n ? py[i] : NAN, tmax + blockIdx.x, tmin + blockIdx.x);
 }
 
+// The flags of k_layout_points before it: on the lattice until a block finds otherwise.
+__global__ void k_layout_flags(int32_t* clat, int32_t* plat) {
+  *clat = 1;
+  if (plat != nullptr) *plat = 1;
+}
+
 // One pass over the centres and the new positions (a block a tile, the centres' tiles
 // first): their half-lattice coordinates and flags (the positions' only if pxy2) and
-// their tiles' extremes.  The last block sets the flags, so that one launch does what a
-// launch each for the flags, the coordinates and the extremes did (2 to 4 us each, all
-// latency).
+// their tiles' extremes, where a launch each for the coordinates and the extremes of both
+// took 2 to 4 us each, all latency.  (A ticket that lets the last block set the flags
+// saves the launch of k_layout_flags, 1466 against 1470 us for a TPS of 255 x 255 vectors,
+// but needs words that are zero before the call, and a plan copied by its header alone has
+// none.)
 __global__ void __launch_bounds__(YB_TILE)
     k_layout_points(const fi_tps_plan* plan, const double* cx, const double* cy, int ncap,
                     int ctiles, int32_t* cxy2, int32_t* clat, double* cb, const double* px,
@@ -548,19 +543,8 @@ __global__ void __launch_bounds__(YB_TILE)
     reinterpret_cast<int2*>(xy2)[i] = c;
   }
   const bool any_off = __syncthreads_or(off) != 0;
+  if (any_off && threadIdx.x == 0) *(set == 0 ? clat : plat) = 0;
   tile_extremes(y, bounds + tile, bounds + (set == 0 ? ctiles : ptiles) + tile);
-  if (threadIdx.x == 0) {
-    PlanWords* w = plan_words(plan);
-    if (any_off) atomicOr(&w->off[set], 1);
-    __threadfence();
-    if (atomicAdd(&w->ticket, 1) == (int)gridDim.x - 1) {
-      __threadfence();
-      *clat = atomicExch(&w->off[0], 0) == 0;
-      const int poff = atomicExch(&w->off[1], 0);
-      if (pxy2 != nullptr) *plat = poff == 0;
-      w->ticket = 0;
-    }
-  }
 }
 
 // In place: running max forward, running min backward over the tiles (one block;
@@ -1653,10 +1637,11 @@ extern "C" int fi_tps_layout(const fi_tps_plan* plan, int nb_subdom, const doubl
   cudaStream_t s = (cudaStream_t)stream;
   const int ctiles = (num_centers + YB_TILE - 1) / YB_TILE;
   const int ptiles = (npts + YB_TILE - 1) / YB_TILE;
+  k_layout_flags<<<1, 1, 0, s>>>(clat, p_given ? nullptr : plat);
   k_layout_points<<<ctiles + ptiles, YB_TILE, 0, s>>>(
       plan, cx, cy, num_centers, ctiles, cxy2, clat, cbounds, px, py, npts, ptiles,
       p_given ? nullptr : pxy2, plat, pbounds);
-  int launched = 3;
+  int launched = 4;
   if (ctiles > YB_SCAN || ptiles > YB_SCAN) {
     k_y_tiles_scan<<<1, 1024, 0, s>>>(ctiles, cbounds, cbounds + ctiles);
     k_y_tiles_scan<<<1, 1024, 0, s>>>(ptiles, pbounds, pbounds + ptiles);

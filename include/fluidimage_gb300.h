@@ -447,8 +447,7 @@ int fi_tps_members(const fi_tps_plan* plan, int nb_subdom, const double* px, con
  * mat_offsets, w_offsets, summary), order (nullable, [nb_subdom]) as in
  * fi_tps_offsets.  No reference counterpart (the
  * bookkeeping of ThinPlateSplineSubdom.__init__ / init_with_new_positions,
- * thin_plate_spline_subdom.py:25-127, 160-206).  Words after the header in the plan's
- * FI_TPS_PLAN_BYTES are used meanwhile: one call at a time on a plan.
+ * thin_plate_spline_subdom.py:25-127, 160-206).  The plan is read only.
  */
 int fi_tps_layout(const fi_tps_plan* plan, int nb_subdom, const double* cx, const double* cy,
                   int num_centers, const double* px, const double* py, int npts, int p_given,
