@@ -1325,6 +1325,7 @@ __global__ void k_tps_blend_centers(const fi_tps_plan* plan_ptr, const double* c
 // 185 -> 103 us; the two fields between the passes of a 2048^2 run 290 -> 130 us.
 constexpr int EVAL_TABLE = 9216;
 constexpr int EVAL_NT = 512;
+constexpr int EVAL_MEMBERS = 3656;  // largest subdomain, by its shared memory
 
 __global__ void __launch_bounds__(EVAL_NT)
     k_tps_eval(const int32_t* counts, const int64_t* offsets, const int32_t* indices,
@@ -1806,7 +1807,9 @@ extern "C" int fi_tps_interpolate(const fi_tps_plan* plan, int nb_subdom, int ma
   cudaStream_t s = (cudaStream_t)stream;
   const int nm = (max_members + 4) & ~1;
   const size_t base = (size_t)nm * (sizeof(float4) + 4 * sizeof(double) + sizeof(int2));
-  FI_REQUIRE(base <= 200 * 1024, "fi_tps_interpolate: subdomain of %d vectors too large",
+  // (3656 centres at 56 bytes and the affine weights in 200 KB; rounded up, 205 KB)
+  FI_REQUIRE(max_members >= 0 && max_members <= EVAL_MEMBERS,
+             "fi_tps_interpolate: subdomain of %d vectors too large",
              max_members);
   FI_REQUIRE(table_entries >= 0 && table_entries <= 16384,
              "fi_tps_interpolate: table_entries %d out of [0, 16384]", table_entries);
