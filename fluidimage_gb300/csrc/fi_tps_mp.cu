@@ -1034,6 +1034,16 @@ __device__ void chol_solve2(const uint4* LP, int m, const float* dsc, float* rx,
   __syncthreads();
 }
 
+// Systems of at most this many unknowns are refined three times at least.  The factor's 22
+// bits contract the error about 4 times less than FP32's 24: what two sweeps leave is above
+// the rounding of B in these.  rms error against FP64, 24 x 26 vectors 8 px apart off the
+// lattice, with two sweeps, with three, and with an FP32 factor: subdomains of 40 vectors
+// 2.0e-12, 3.8e-13, 7.8e-13; of 60 6.9e-12, 6.6e-13, 2.5e-12.  From 100 vectors on (most
+// above 140 unknowns) two sweeps that pass are no worse than with the FP32 factor (0.91 of
+// its error over steps of 4 to 32 px, smoothing 0.5 to 5).  The third sweep: 255 x 255
+// vectors in subdomains of 40 885 -> 979 us.
+constexpr int SETTLE = 128;
+
 // Shared-memory layout of k_tps_solve_mp for subdomains of at most n centres.
 struct MpLayout {
   int np;        // n rounded up to 32
@@ -1472,8 +1482,8 @@ __global__ void __launch_bounds__(NT, 512 / NT)
       }
       __syncthreads();
     }
-    // refine z (B z = g): FP32 Cholesky solves, double-float residuals
-    bool conv = false;
+    // refine z (B z = g): solves with the factor, double-float residuals
+    bool conv = false, near = false;
     double prev = INFINITY;
     for (int it = 0; it < max_refine; ++it) {
       if (z_zero) {  // z = 0: rho = g
@@ -1514,12 +1524,15 @@ __global__ void __launch_bounds__(NT, 512 / NT)
         break;
       }
       if (it >= 1) {
-        // contraction of the FP32-preconditioned refinement, estimated from the last
-        // two corrections; the remaining error is about contraction * dmax.  4e-11 of z:
-        // the field then carries the rounding of B, not the refinement's (2e-11 to 8e-11
-        // relative against FP64 LU; 4e-11 to 1.6e-10 at 1e-10, for 1-2 % less time)
+        // contraction of the preconditioned refinement, estimated from the last two
+        // corrections; the remaining error is about contraction * dmax.  4e-11 of z: the
+        // field then carries the rounding of B, not the refinement's (2e-11 to 8e-11
+        // relative against FP64 LU; 4e-11 to 1.6e-10 at 1e-10, for 1-2 % less time).  In
+        // small systems the rounding of B is below that, so they take three sweeps at
+        // least (SETTLE).
         const double rho = dmax / prev;
-        if (rho < 0.1 && rho * dmax <= 4e-11 * zmax) {
+        near = near || (rho < 0.1 && rho * dmax <= 4e-11 * zmax);
+        if (near && it >= (m <= SETTLE ? 2 : 1)) {
           conv = true;
           break;
         }
