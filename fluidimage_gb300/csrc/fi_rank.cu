@@ -620,10 +620,16 @@ static bool takes_minmax_tile(int dtype, int st, int sy, int sx, int rank) {
 // k_rank_planes or k_rank_select_tile (both exact).  A thread of the second counts its
 // window's values for every bit: 17.5 ns per value and bit, 0.2 ps per pixel, value and bit
 // once the chip is full.  A warp of the first takes a 32 x 32 tile in a time that hardly
-// depends on the window and not on how many tiles there are while all are resident (16, 8
+// depends on the window and not on how many tiles there are while all are resident (16, 12
 // or 4 warps an SM by the planes' size): 70 to 390 us for 8 bits, 260 to 1260 for 16, 1440
-// to 1900 for 32, less for images than for noise and for large windows; the lines lie at
-// the values below.  Median, us, planes and select, particle image / noise:
+// to 1900 for 32, less for images than for noise and for large windows.  Which kernel is
+// faster near the line depends on the image, which the rule does not see: the values below
+// lie between particle images and noise.  Past 16, 8 or 4 tiles an SM the time is taken to
+// grow with the tiles; for 16 bits that is before they fill the chip (1216 of 1824 resident
+// tiles): at 2048^2, 4096 tiles, particle images take 2.0 times what 1024 tiles take and
+// noise 2.9 times, and a line from 1824 on would give 10 to 12 px windows to the planes
+// (12 x 12: 1228 against 1695 us, noise 3444 against 2231).
+// Median, us, planes and select, particle image / noise:
 //   u8  512^2  5 x 5: 160 and 34 / 343 and 33;      30 x 30: 78 and 476 / 160 and 476
 //   u16 512^2  5 x 5: 563 and 46 / 1208 and 56;     30 x 30: 344 and 703 / 1029 and 934
 //   u16 2048^2 9 x 9: 1355 and 1113 / 3557 and 1458; 30 x 30: 726 and 9212 / 3058 and 12251
@@ -631,11 +637,11 @@ static bool takes_minmax_tile(int dtype, int st, int sy, int sx, int rank) {
 static bool planes_pay(int dtype, int nt, int ny, int nx, int sy, int sx) {
   const int bits = dtype == FI_PRE_U8 ? 8 : dtype == FI_PRE_U16 ? 16 : 32;
   const double tile_us = bits == 8 ? 180.0 : bits == 16 ? 600.0 : 1700.0;
-  const double resident = 152.0 * 128 / bits;
+  const double full = (double)num_sms() * 128 / bits;  // 16, 8, 4 tiles an SM
   const double tiles = (double)nt * ((ny + RP_T - 1) / RP_T) * ((nx + RP_T - 1) / RP_T);
   const double counts = (double)sy * sx * bits, pixels = (double)nt * ny * nx;
   const double select_us = counts * (pixels * 2.03e-7 > 0.0175 ? pixels * 2.03e-7 : 0.0175);
-  return select_us > tile_us * (tiles > resident ? tiles / resident : 1.0);
+  return select_us > tile_us * (tiles > full ? tiles / full : 1.0);
 }
 static bool takes_time(int dtype, int nt, int st, int sy, int sx) {
   return sy == 1 && sx == 1 && st > 1 &&

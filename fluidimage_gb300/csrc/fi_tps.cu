@@ -1823,7 +1823,7 @@ extern "C" int fi_tps_interpolate(const fi_tps_plan* plan, int nb_subdom, int ma
   if (max_new_members > 0) {
     // wide blocks share a large table between more warps; narrow ones where a subdomain's
     // positions fill few of them
-    const int nt = (int64_t)nb_subdom * (max_new_members / EVAL_NT) >= 152 ? EVAL_NT : 256;
+    const int nt = (int64_t)nb_subdom * (max_new_members / EVAL_NT) >= num_sms() ? EVAL_NT : 256;
     dim3 grid((max_new_members + nt - 1) / nt, nb_subdom);
     k_tps_eval<<<grid, nt, smem, s>>>(
         counts, offsets, indices, w_offsets, weights, cx, cy, ncounts, noffsets, nindices, ncoefs,
