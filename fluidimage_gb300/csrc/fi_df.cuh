@@ -25,28 +25,15 @@ __device__ __forceinline__ float2 df_add(float2 a, float2 b) {
   return make_float2(hi, __fsub_rn(lo, __fsub_rn(hi, s)));
 }
 
-// (sh, sl) += b * z (the lo * lo term, 2^-48 relative, is dropped)
-__device__ __forceinline__ void df_mac(float2 b, float2 z, float& sh, float& sl) {
-  const float p = __fmul_rn(b.x, z.x);
-  float e = __fmaf_rn(b.x, z.x, -p);
-  e = __fmaf_rn(b.x, z.y, e);
-  e = __fmaf_rn(b.y, z.x, e);
-  const float t = __fadd_rn(sh, p);
-  const float bb = __fsub_rn(t, sh);
-  const float err = __fadd_rn(__fsub_rn(sh, __fsub_rn(t, bb)), __fsub_rn(p, bb));
-  sl = __fadd_rn(sl, __fadd_rn(err, e));
-  sh = t;
-}
-
 // a - b of two pairs (an exact product by -1 in a fused multiply-add: one packed
 // instruction, where the negation of a pair would take its own)
 __device__ __forceinline__ float2 df_sub2(float2 a, float2 b) {
   return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
 }
 
-// Two independent df_mac in the lanes of float2 pairs, with packed FP32x2
-// instructions (each lane rounds exactly as df_mac):
-// (sh.x, sl.x) += b * (zh.x + zl.x) and (sh.y, sl.y) += b * (zh.y + zl.y).
+// (sh.x, sl.x) += b * (zh.x + zl.x) and (sh.y, sl.y) += b * (zh.y + zl.y), b = b.x + b.y, by
+// error-free products and sums in packed FP32x2 instructions (the lo * lo terms, 2^-48
+// relative, are dropped).
 __device__ __forceinline__ void df_mac_x2(float2 b, float2 zh, float2 zl, float2& sh,
                                           float2& sl) {
   const float2 bh = make_float2(b.x, b.x), nbh = make_float2(-b.x, -b.x);

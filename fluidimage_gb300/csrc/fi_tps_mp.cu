@@ -1067,10 +1067,13 @@ struct MpLayout {
 // One block per subdomain.  Status per subdomain: 0 solved here, 1 needs the FP64
 // LU fallback (rank-deficient P, Cholesky breakdown or no convergence).
 //
-// Buffers per subdomain (offset mat_off, a multiple of 4 elements): matrices holds
-// B22 = (Q^T A Q)[3:, 3:] as (hi, lo) float pairs, both triangles, leading
-// dimension mp = m rounded up to 4; matrices32 holds the tiles of its Cholesky factor
-// (chol_factor; in shared memory for small subdomains).
+// Buffers per subdomain (offset mat_off, a multiple of 4 elements; (m + 6)^2 doubles and as
+// many floats): matrices holds B22 = (Q^T A Q)[3:, 3:] as (hi, lo) float pairs, the 32 x 32
+// tiles of its lower half (BPairs), and behind them, from 7 tile rows on, the residual's
+// partial sums (residual_part_bytes: tiles and sums of T rows are below (32 T - 25)^2 pairs,
+// the smallest slot with T rows, for T >= 7); matrices32 holds the tiles of its Cholesky
+// factor (chol_factor).  Up to 32 SMALL_T unknowns B22 is whole, both triangles, leading
+// dimension mp = m rounded up to 4, and the factor in shared memory.
 template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT)
     k_tps_solve_mp(const fi_tps_plan* plan_ptr, const double* cx, const double* cy,
