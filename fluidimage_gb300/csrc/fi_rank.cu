@@ -537,10 +537,21 @@ __global__ void k_rank_select(const void* in, int dtype, int64_t nt, int64_t ny,
 // k_rank_planes takes, by tiles: a block stages its output tile plus the window halo
 // (boundary extension applied once per staged element) as 32-bit keys in shared memory,
 // then each thread runs the radix select over its window there; the select starts at the
-// highest key bit set in the tile (higher bits are zero for every staged value).
+// highest key bit set in the tile (higher bits are zero for every staged value).  Bound by
+// the loads of the loop over the window, which runs slower with the result's conversion and
+// subtraction in the same function (put_apart): medians of 1024^2 f32, 7, 10 and 15 px 567,
+// 887 and 1938 us so, 479, 842 and 1750 us apart.
+// NARROW (windows up to 5 px wide): the values with the prefix and a 0 at bit b as the range
+// [prefix, prefix + 2^b), one comparison a value: 1024^2 f32 3 px 148 -> 138 us, 5 px 278 and
+// 277; from 7 px on the form of two tests is faster (10 px 888 against 842 us).
 constexpr int RS_TX = 32, RS_TY = 16;
 constexpr int RS_MAX_SMEM = 96 * 1024;
 
+static __device__ __noinline__ void put_apart(const RankOut& ro, int64_t e, uint32_t key) {
+  ro.put(e, key);
+}
+
+template <bool NARROW>
 __global__ void __launch_bounds__(RS_TX * RS_TY)
     k_rank_select_tile(const void* in, int dtype, int64_t ny, int64_t nx, int sy, int sx,
                        int rank, int mode, uint32_t ckey, RankOut ro) {
@@ -578,10 +589,7 @@ __global__ void __launch_bounds__(RS_TX * RS_TY)
     int zeros = 0;
     for (int c = 0; c < sy; ++c) {
       const uint32_t* row = patch + (threadIdx.y + c) * pw + threadIdx.x;
-      if (sx <= 15) {
-        // the values with the prefix and a 0 at bit b are those in [prefix, prefix + 2^b):
-        // medians of 1024^2 u16, 5 x 5, 7 x 7, 13 x 13: 134, 226, 557 -> 119, 199, 523 us;
-        // wider rows run faster in the form below (16 x 16: 697 against 750)
+      if (NARROW) {
 #pragma unroll 4
         for (int d = 0; d < sx; ++d) zeros += row[d] - prefix < (1u << b) ? 1 : 0;
       } else {
@@ -596,7 +604,7 @@ __global__ void __launch_bounds__(RS_TX * RS_TY)
       prefix |= (1u << b);
     }
   }
-  ro.put((t * ny + y) * nx + x, prefix);
+  put_apart(ro, (t * ny + y) * nx + x, prefix);
 }
 
 __global__ void k_subtract_weighted(const void* img, const void* filt, int64_t count, Subtract sub,
@@ -695,6 +703,19 @@ static int launch_planes(const void* in, int dtype, int nt, int ny, int nx, int 
   return check_launch("fi_rank_filter");
 }
 
+template <bool NARROW>
+static int launch_select(const void* in, int dtype, int nt, int ny, int nx, int sy, int sx,
+                         int rank, int mode, uint32_t ckey, const RankOut& ro, size_t smem,
+                         cudaStream_t s) {
+  static SmemLimit limit;
+  FI_CUDA_TRY(raise_smem_limit(k_rank_select_tile<NARROW>, smem, limit));
+  const dim3 grid((unsigned)((nx + RS_TX - 1) / RS_TX), (unsigned)((ny + RS_TY - 1) / RS_TY),
+                  (unsigned)nt);
+  k_rank_select_tile<NARROW><<<grid, dim3(RS_TX, RS_TY), smem, s>>>(in, dtype, ny, nx, sy, sx,
+                                                                    rank, mode, ckey, ro);
+  return check_launch("fi_rank_filter");
+}
+
 static int rank_filter(const void* in, int dtype, int nt, int ny, int nx, int st, int sy, int sx,
                        int rank, int mode, double cval, void* scratch, const RankOut& ro,
                        cudaStream_t s) {
@@ -771,15 +792,11 @@ static int rank_filter(const void* in, int dtype, int nt, int ny, int nx, int st
     return launch_planes<32>(in, dtype, nt, ny, nx, sy, sx, rank, mode, (uint32_t)ckey, ro, s);
   }
   const size_t tile_smem = (size_t)(RS_TX + sx - 1) * (RS_TY + sy - 1) * sizeof(uint32_t);
-  if (tiled && st == 1 && dtype != FI_PRE_F64 && tile_smem <= RS_MAX_SMEM) {
-    static SmemLimit limit;
-    FI_CUDA_TRY(raise_smem_limit(k_rank_select_tile, tile_smem, limit));
-    const dim3 grid((unsigned)((nx + RS_TX - 1) / RS_TX), (unsigned)((ny + RS_TY - 1) / RS_TY),
-                    (unsigned)nt);
-    k_rank_select_tile<<<grid, dim3(RS_TX, RS_TY), tile_smem, s>>>(
-        in, dtype, ny, nx, sy, sx, rank, mode, (uint32_t)ckey, ro);
-    return check_launch("fi_rank_filter");
-  }
+  if (tiled && st == 1 && dtype != FI_PRE_F64 && tile_smem <= RS_MAX_SMEM)
+    return sx <= 5 ? launch_select<true>(in, dtype, nt, ny, nx, sy, sx, rank, mode, (uint32_t)ckey,
+                                         ro, tile_smem, s)
+                   : launch_select<false>(in, dtype, nt, ny, nx, sy, sx, rank, mode,
+                                          (uint32_t)ckey, ro, tile_smem, s);
   k_rank_select<<<g, 256, 0, s>>>(in, dtype, nt, ny, nx, st, sy, sx, rank, mode, ckey, ro);
   return check_launch("fi_rank_filter");
 }
