@@ -162,12 +162,18 @@ def _rank_args(img, window, rank_kind, percentile, mode, cval):
         raise RuntimeError(f"boundary mode not supported: {mode}")
     dtype = _dtype_of(x)
     dt = _DT[dtype]
-    if dt in (L.PRE_F32, L.PRE_F64) and bool(torch.isnan(x).any()):
-        raise ValueError("rank filters of images with NaN are not provided")
     scratch = None
     if L.load().fi_rank_needs_scratch(dt, nt, ny, st, sy, sx, r):
         scratch = torch.empty(2 * x.numel(), dtype=torch.int64, device=x.device)
     return x, dtype, (dt, nt, ny, nx, st, sy, sx, r, L.MODES[mode], float(cval)), scratch
+
+
+def _refuse_nan(x):
+    """Waits for the GPU where the image can hold NaN: the last thing before a launch, so
+    that no host work is left between the two."""
+    torch = _torch()
+    if x.is_floating_point() and bool(torch.isnan(x).any()):
+        raise ValueError("rank filters of images with NaN are not provided")
 
 
 def rank_filter(img, window, rank_kind, percentile=None, mode="reflect", cval=0.0):
@@ -175,6 +181,7 @@ def rank_filter(img, window, rank_kind, percentile=None, mode="reflect", cval=0.
     (nt, ny, nx) over the box ``window`` = (st, sy, sx); output in the input dtype."""
     x, _, args, scratch = _rank_args(img, window, rank_kind, percentile, mode, cval)
     out = _torch().empty_like(x)
+    _refuse_nan(x)
     L.check(L.load().fi_rank_filter(L.ptr(x), L.ptr(out), *args, L.ptr(scratch),
                                     L.stream_handle()), "fi_rank_filter")
     return out
@@ -194,6 +201,7 @@ def _rank_subtract(img, window, rank_kind, percentile, weight, clamp, mode="refl
     if out_dt not in _DT:
         raise TypeError(f"result dtype {out_dt} not supported")
     out = _empty(tuple(x.shape), out_dt, x.device)
+    _refuse_nan(x)
     L.check(L.load().fi_rank_subtract(L.ptr(x), L.ptr(out), *args, float(weight), _DT[out_dt],
                                       int(clamp), L.ptr(scratch), L.stream_handle()),
             "fi_rank_subtract")
