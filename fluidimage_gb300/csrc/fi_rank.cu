@@ -164,13 +164,14 @@ inline size_t time_bytes(int nt, int st) {
   return (size_t)nt * TIME_NT * sizeof(W) + (size_t)(nt + st) * sizeof(int);
 }
 
-// E: bits of a packed element (8, 16), or 0: one key per word
-template <typename W, int E>
+// E: bits of a packed element (8, 16), or 0: one key per word; SPLIT: frames dealt to
+// blockIdx.y (with the general bounds the unsplit launch is 2 % slower)
+template <typename W, int E, bool SPLIT>
 __global__ void __launch_bounds__(TIME_NT)
     k_time_rank(const void* in, int dtype, int nt, int64_t npix, int st, int rank, int mode,
                 uint64_t ckey, int span, RankOut ro) {
   constexpr int V = E == 8 ? 4 : E == 16 ? 2 : 1;
-  const int t_lo = blockIdx.y * span, t_hi = min(nt, t_lo + span);
+  const int t_lo = SPLIT ? blockIdx.y * span : 0, t_hi = SPLIT ? min(nt, t_lo + span) : nt;
   extern __shared__ __align__(16) unsigned char tm_smem[];
   W* col = reinterpret_cast<W*>(tm_smem) + threadIdx.x;
   int* at = reinterpret_cast<int*>(reinterpret_cast<W*>(tm_smem) + (size_t)nt * TIME_NT);
@@ -670,24 +671,34 @@ static int launch_minmax_tile(const void* in, int dtype, int nt, int ny, int nx,
   return check_launch("fi_rank_filter");
 }
 
+template <typename W, int E, bool SPLIT>
+static int launch_time_parts(const void* in, int dtype, int nt, int64_t npix, int st, int rank,
+                             int mode, uint64_t ckey, int64_t blocks, int span, const RankOut& ro,
+                             cudaStream_t s) {
+  const size_t smem = time_bytes<W>(nt, st);
+  static SmemLimit limit;
+  FI_CUDA_TRY(raise_smem_limit(k_time_rank<W, E, SPLIT>, smem, limit));
+  const int64_t most = 64 * (int64_t)num_sms();
+  const dim3 grid((unsigned)(blocks < most ? blocks : most), (unsigned)((nt + span - 1) / span));
+  k_time_rank<W, E, SPLIT><<<grid, TIME_NT, smem, s>>>(in, dtype, nt, npix, st, rank, mode, ckey,
+                                                       span, ro);
+  return check_launch("fi_rank_filter");
+}
+
 template <typename W, int E>
 static int launch_time(const void* in, int dtype, int nt, int64_t npix, int st, int rank, int mode,
                        uint64_t ckey, const RankOut& ro, cudaStream_t s) {
-  const size_t smem = time_bytes<W>(nt, st);
-  static SmemLimit limit;
-  FI_CUDA_TRY(raise_smem_limit(k_time_rank<W, E>, smem, limit));
   const int V = E == 8 ? 4 : E == 16 ? 2 : 1;
-  const int64_t blocks = (npix / V + TIME_NT - 1) / TIME_NT, sms = num_sms();
+  const int64_t blocks = (npix / V + TIME_NT - 1) / TIME_NT;
   // blocks resident at once, by shared memory (228 KB an SM, 1 KB of it per block) and threads
-  const int64_t per_sm = 228 * 1024 / (int64_t)(smem + 1024);
-  const int64_t resident = sms * (per_sm < 2048 / TIME_NT ? per_sm : 2048 / TIME_NT);
+  const int64_t per_sm = 228 * 1024 / (int64_t)(time_bytes<W>(nt, st) + 1024);
+  const int64_t resident = num_sms() * (per_sm < 2048 / TIME_NT ? per_sm : 2048 / TIME_NT);
   const int64_t parts = resident / blocks < nt ? resident / blocks : nt;
-  const int span = parts > 1 ? (int)((nt + parts - 1) / parts) : nt;
-  const dim3 grid((unsigned)(blocks < sms * 64 ? blocks : sms * 64),
-                  (unsigned)((nt + span - 1) / span));
-  k_time_rank<W, E><<<grid, TIME_NT, smem, s>>>(in, dtype, nt, npix, st, rank, mode, ckey, span,
-                                                ro);
-  return check_launch("fi_rank_filter");
+  if (parts <= 1)
+    return launch_time_parts<W, E, false>(in, dtype, nt, npix, st, rank, mode, ckey, blocks, nt,
+                                          ro, s);
+  return launch_time_parts<W, E, true>(in, dtype, nt, npix, st, rank, mode, ckey, blocks,
+                                       (int)((nt + parts - 1) / parts), ro, s);
 }
 
 template <int BITS>
