@@ -58,8 +58,9 @@ class _Arrays:
     pinned buffer (one per thread, at most ``STAGE_MAX``), which the GPU reads and writes
     over its link to the host, so that a call is a launch and one synchronisation: a
     32 px window through correlation, peak and subpixel fit 585 -> 111 us.  Larger calls
-    go through device memory (21 windows of 64 px, 1 MB: 180 us, pinned 99; 256 of 32
-    px, 3 MB: 744 and 220), so that the buffer stays bounded.
+    go through device memory, the inputs array by array and the outputs in one copy, so
+    that the buffer stays bounded (planes and peaks of 256 windows of 32 px 424 us, of
+    1024 of 48 px 1302; with a copy for each array 540 and 1449).
     """
 
     def __init__(self, specs):
@@ -72,7 +73,8 @@ class _Arrays:
             total += -(-nbytes // 16) * 16
         total = max(total, 16)
         self.stream = torch.cuda.current_stream()
-        self.device = None
+        self.host = self.device = None
+        self.first = 0  # where the host's bytes begin
         if total <= STAGE_MAX:
             stage = getattr(_STAGE, "stage", None)
             if stage is None or stage[0].numel() < total:
@@ -80,34 +82,40 @@ class _Arrays:
                 stage = _STAGE.stage = buf, buf.numpy(), buf.data_ptr()
             _, self.host, base = stage
         else:
-            self.host = np.empty(total, dtype=np.uint8)
             self.device = torch.empty(total, dtype=torch.uint8, device=_dev())
             base = self.device.data_ptr()
         self.ptr = [base + span[0] for span in self.spans]
 
     def view(self, i):
         at, nbytes, dtype, shape = self.spans[i]
-        return self.host[at:at + nbytes].view(dtype).reshape(shape)
+        if at < self.first:  # an input in device memory, as the kernels left it
+            raw = self.device[at:at + nbytes].cpu().numpy()
+        else:
+            raw = self.host[at - self.first:at - self.first + nbytes]
+        return raw.view(dtype).reshape(shape)
 
     def start(self, *inputs):
         """Fills the first arrays; what the library needs before the launch."""
         for i, array in enumerate(inputs):
-            self.view(i)[...] = array
-        if self.device is not None:
-            import torch
+            if self.device is None:
+                self.view(i)[...] = array
+            else:
+                import torch
 
-            end = self.spans[len(inputs)][0]
-            self.device[:end].copy_(torch.from_numpy(self.host[:end]))
+                at, nbytes, dtype, _ = self.spans[i]
+                raw = np.ascontiguousarray(array, dtype=dtype).reshape(-1).view(np.uint8)
+                self.device[at:at + nbytes].copy_(torch.from_numpy(raw))
+                self.first = self.spans[i + 1][0]
         return self.stream.cuda_stream
 
     def finish(self):
-        if self.device is not None:
-            self.host = self.device.cpu().numpy()
-        else:
+        if self.device is None:
             self.stream.synchronize()
+        else:  # the outputs in one copy, the caller's own
+            self.host = self.device[self.first:].cpu().numpy()
 
     def get(self, i):
-        return self.view(i).copy()
+        return self.view(i).copy() if self.device is None else self.view(i)
 
 
 _F64, _F32, _I32, _U8 = (np.dtype(t) for t in ("f8", "f4", "i4", "u1"))
