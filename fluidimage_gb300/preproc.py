@@ -510,8 +510,11 @@ def adaptive_threshold(img, window_size=5, offset=0):
     return out - offset
 
 
-#: largest filter radius of fi_sharpen
+#: largest filter radius of fi_sharpen, and its largest images: the frames and the tiles of
+#: 32 rows are launch dimensions
 SHARPEN_MAX_RADIUS = 32
+SHARPEN_MAX_FRAMES = 65535
+SHARPEN_MAX_ROWS = 65535 * 32
 
 
 @_per_image
@@ -526,7 +529,8 @@ def sharpen(img, sigma1=3.0, sigma2=1.0, alpha=30.0):
         nt, ny, nx = x.shape
         w1, r1 = _gauss_weights(sigma1)
         w2, r2 = _gauss_weights(sigma2)
-        if max(r1, r2) <= SHARPEN_MAX_RADIUS and nt <= 65535:
+        if (max(r1, r2) <= SHARPEN_MAX_RADIUS and nt <= SHARPEN_MAX_FRAMES
+                and ny <= SHARPEN_MAX_ROWS):
             blurred = _torch().empty_like(x)
             out = _empty((nt, ny, nx), np.float64, x.device)
             L.check(L.load().fi_sharpen(L.ptr(x), L.ptr(out), L.ptr(blurred), _DT[dtype], nt, ny,
