@@ -115,6 +115,7 @@ __device__ __forceinline__ const void* image_of(const void* im, int b, int H, in
 }
 
 // 2048^2 float32: 50 -> 19 us per image (a binary search of both axes for every pixel).
+// Bound by the latency of the samples' loads: issue 59 % of the slots, DRAM 11 %.
 template <int DT>
 __global__ void __launch_bounds__(WT_X * 8)
     k_warp(const float* __restrict__ fld, const float* __restrict__ xn, int nx,
@@ -376,7 +377,8 @@ __global__ void __launch_bounds__(32 * WPB)
 // a lane adds dL/d(u, v) weighted by (1 - ty) and ty (its tx is constant); where the cell
 // changes, and at the end of its rows, the four sums times (1 - tx) and tx are reduced over
 // the lanes of each cell by shuffles and added to global memory by one lane.  2048^2
-// float32: 108 -> 32 us per image (eight reductions per row of 32 pixels before).
+// float32: 108 -> 32 us per image (eight reductions per row of 32 pixels before).  Bound by
+// the samples' loads as k_warp: issue 61 % of the slots, DRAM 13 %.
 template <int DT>
 __global__ void __launch_bounds__(WT_X * 8)
     k_warp_bwd(const float* __restrict__ fld, const float* __restrict__ xn, int nx,

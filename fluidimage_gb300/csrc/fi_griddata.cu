@@ -975,8 +975,10 @@ __device__ __forceinline__ bool take_query(const GdArgs& a, const Group<G>& g, Q
   return done;
 }
 
-// Bound by the instructions of a query's exact predicates and, at the borders and
-// around holes, by the few queries whose window grows (up to C(64, 3) triples each).
+// Bound by the dependent instructions of a query's exact predicates at 16 warps an SM
+// (registers; issue 22 and 39 % of the slots for 8 900 and 36 000 queries) and, at the
+// borders and around holes, by the few queries whose window grows (up to C(64, 3) triples
+// each).
 // Eight lanes take a query: they share the nodes of a window (each loaded once, in
 // registers up to two steps) and the triples, and every decision is the group's.  The
 // block's queries that need more than GD_QUICK steps are then taken by whole warps (the

@@ -62,7 +62,8 @@ __global__ void k_gauss_axis(const void* in, void* out, int dtype, int nt, int n
 // constant area): then the line is summed again in float64, in scipy's order.  Weights
 // outside [0, 1] take that path for every pixel.
 // SHARPEN: the image is the blurred one, and out = image + alpha (image - filtered).
-// 2048^2 u16, sigma 3 then 1 and the combination: 1552 -> 147 us.
+// 2048^2 u16, sigma 3 then 1 and the combination: 1552 -> 147 us (94 and 56; issue 66 % of
+// the slots, its stalls the math pipes' throttle; L1 52 and 38 %, DRAM 1 to 2 %).
 // Small images take tiles of fewer rows (gauss_tile_rows), so that they fill the chip:
 // whole calls of constant areas (every pixel on the float64 path), sigma 8 twice, 64 x 64
 // 420 -> 137 us, 227 x 379 428 -> 218 us (one pixel per thread in float64: 206 and 281).

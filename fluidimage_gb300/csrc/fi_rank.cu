@@ -41,7 +41,8 @@ struct RankOut {
 // the window) in place of one buffer into the other, and the window as two overlapping
 // runs of p.  A 30 x 30 window takes 5 + 5 minima per element instead of 30 + 30 loads of
 // 64-bit keys from memory in three passes: 4 frames of 512^2 u8 with the subtraction
-// 140 -> 33 us a call (host-bound).
+// 140 -> 36 us a call.  The kernel takes most of it, by the latency of its steps (a barrier
+// between each two of 12): warps 39 % of the most, issue 46 % of the slots, DRAM 0.4 %.
 constexpr int MM_TX = 64, MM_TY = 32, MM_NT = 256;
 constexpr size_t MM_MAX_SMEM = 160 * 1024;
 
@@ -151,7 +152,7 @@ __global__ void k_keys_out(const uint64_t* k, int64_t count, RankOut ro) {
 // maxima by packed instructions, other ranks by a radix select over the bits in which the
 // pixel's frames differ.  The minimum over 8 frames of 2048^2 u16 with the subtraction
 // 1666 -> 80 us (three axis passes over 64-bit keys, a conversion and the subtraction
-// before).  A thread's output frames are a serial chain, so where the pixels do not fill
+// before); bound by issue, 84 % of the slots, with DRAM at 43 %.  A thread's output frames are a serial chain, so where the pixels do not fill
 // the chip the frames are dealt to blockIdx.y, `span` each (every block reads all frames):
 // medians over all frames, whole call, 95 frames of 16^2 u8 5085 -> 71 us, 90 of 48^2 u16
 // 5022 -> 127 us, 40 of 64^2 f32 910 -> 144 us (k_rank_select, one thread per value: 342,
@@ -290,7 +291,9 @@ __global__ void __launch_bounds__(TIME_NT)
 // Pixels of a tile share prefixes (a median varies slowly), and nodes with few pixels are
 // finished one pixel at a time, the window's rows over the lanes (one reduction per bit),
 // so that even unrelated values cost at most that.  2048^2 u16, 30 x 30: 9160 -> 524 us
-// (a thread per pixel counting its 900 values for every bit before).
+// (a thread per pixel counting its 900 values for every bit before).  Bound by the latency
+// of a warp's dependent steps: shared memory leaves 12 warps an SM at 16 bits, issue 29 % of
+// the slots, L1 23 %.
 constexpr int RP_T = 32;            // tile edge
 constexpr int RP_ROWS = 64;         // rows of the tile with its halo, at most
 constexpr int RP_LD = RP_ROWS + 1;  // row stride of the planes (a row's planes are written
