@@ -391,6 +391,12 @@ __device__ __forceinline__ bool same_weights(const int (&ti)[3], const I (&to)[3
 constexpr int GD_THREADS = 128;  // a block
 constexpr int GD_LANES = 8;      // lanes a query, while its window is small
 constexpr int GD_QUICK = 2;      // steps of those windows (then a warp takes the query)
+// Up to this many queries an SM a block has four of them, one warp's groups: all blocks are
+// resident at once (four an SM, by registers), and each query that is left has a warp of its
+// own.  With 16 a block four follow each other on a warp while most SMs are idle: 414
+// queries around 5 vectors of a 2 x 23 grid 99 us so, 47 with four (a thread a query: 65),
+// 464 of a full 4 x 29 grid 74 and 44; equal where no query is left, and from 2432 on.
+constexpr int GD_FEW = 16;
 
 // The groups of a warp go in step: every collective is the warp's (a group's own mask
 // would have its groups run one after the other), so what a group decides for itself is
@@ -987,15 +993,15 @@ __device__ __forceinline__ bool take_query(const GdArgs& a, const Group<G>& g, Q
 // thread a query, 0.51 ms with eight lanes throughout, 0.30 ms with a warp throughout,
 // 0.22 ms as here; the same grid with 2 % holes 260, 79, 193 and 81 us; 255 x 255 with
 // 3 % holes, 261 121 queries: 27, 7.8, 2.9 and 2.4 ms.
-__global__ void __launch_bounds__(GD_THREADS) k_gd_interp(GdArgs a) {
+__global__ void __launch_bounds__(GD_THREADS) k_gd_interp(GdArgs a, int per_block) {
   __shared__ unsigned long long s_near[GD_THREADS / GD_LANES][GD_MAXC];
   __shared__ Query s_left[GD_THREADS / GD_LANES];
   __shared__ int s_nleft;
   if (threadIdx.x == 0) s_nleft = 0;
   __syncthreads();
   const int slot = threadIdx.x / GD_LANES;
-  const int q = blockIdx.x * (GD_THREADS / GD_LANES) + slot;
-  {
+  const int q = blockIdx.x * per_block + slot;
+  if (slot < per_block) {  // whole warps
     const Group<GD_LANES> g(threadIdx.x);
     Query qs{q < a.npts ? q : -1, 1, {-1, -1, -1}};
     if (!take_query(a, g, qs, GD_QUICK, s_near[slot]) && g.lane == 0)
@@ -1053,8 +1059,8 @@ extern "C" int fi_griddata(const double* cx, const double* cy, const float* ux, 
   int m2 = 64;
   while (m2 < next) m2 <<= 1;
   k_gd_hull<<<1, min(1024, max(64, m2 / 2)), 0, s>>>(nx, ny, m2, left, right, hull_n);
-  constexpr int per_block = GD_THREADS / GD_LANES;
-  k_gd_interp<<<(npts + per_block - 1) / per_block, GD_THREADS, 0, s>>>(a);
+  const int per_block = npts <= GD_FEW * num_sms() ? 32 / GD_LANES : GD_THREADS / GD_LANES;
+  k_gd_interp<<<(npts + per_block - 1) / per_block, GD_THREADS, 0, s>>>(a, per_block);
   return check_launch("fi_griddata", 4);
 }
 
